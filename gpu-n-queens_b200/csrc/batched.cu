@@ -59,6 +59,8 @@ constexpr uint32_t kNoItem = 0xFFFFFFFFu;
 // than 16 (the per-round checks cost more than the idle lanes they save), 48 another 0.75%,
 // and 64 is slower again.
 constexpr int kUnroll = NQB_BATCHED_UNROLL;
+constexpr int kRefresh = 24;  // steps between refreshes of the lanes' sentinels
+static_assert(kRefresh <= kMaxParkedSteps, "a parked lane would pop past its sentinel");
 constexpr uint32_t kEpoch = (1u << 27) / kUnroll;  // rounds between folds: 31 nodes x kUnroll x kEpoch < 2^32
 constexpr uint32_t kDonateEvery = 16;        // rounds between a busy warp's looks at the hungry count
 // The spread instance (launches with fewer items than lanes) looks 8x less often.  Measured on
@@ -143,11 +145,11 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
     s.sols = 0;
     s.nodes = 0;
     s.err = 0;
+    s.placed = 0;
     uint32_t weight = 0, item = kNoItem;
     unsigned long long piece_sols = 0, piece_nodes = 0;  // folded lane counters of the current piece
     unsigned long long total = 0, total_nodes = 0;
     unsigned long long placed64 = 0, rounds64 = 0;       // LANES builds
-    uint32_t placed = 0;
     bool bad = false, qempty = false, stalled = false;
     uint32_t epoch = kEpoch, rounds = 0;
 
@@ -364,15 +366,15 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
             piece_sols += s.sols;
             piece_nodes += s.nodes;
             s.sols = s.nodes = 0;
-            placed64 += placed;
-            placed = 0;
+            placed64 += s.placed;
+            s.placed = 0;
             epoch = kEpoch;
         }
         if (LANES) ++rounds64;
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const StepInfo si = search_step<kStride>(s, base, top);
-            if (LANES) placed += (si.placed != 0u);
+        for (int u = 0; u < kUnroll; u += 2) {
+            if (u % kRefresh == 0) refresh_sentinel(base);
+            search_two_steps<kStride, LANES>(s, base, top);
         }
     }
 
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
     const unsigned any_bound = __any_sync(kFull, s.err != 0);  // checked builds only
     const unsigned any_stall = __any_sync(kFull, stalled);
     if (LANES) {
-        placed64 = warp_sum_u64(placed64 + placed);
+        placed64 = warp_sum_u64(placed64 + s.placed);
         if (lane == 0) {
             atomicAdd(a.lane_stats + 0, placed64);
             atomicAdd(a.lane_stats + 1, 32ull * kUnroll * rounds64);

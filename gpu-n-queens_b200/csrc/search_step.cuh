@@ -4,24 +4,27 @@
 // A lane's search state is four 32-bit words kept in registers:
 //   avail  candidate columns of the current row still to be searched below
 //   nc     columns without a queen
-//   l, r   columns of the current row attacked along the two diagonals
+//   l      columns of the NEXT row attacked along the left diagonals from above this row
+//   r      columns of this row attacked along the right diagonals
 // plus `sp`, the shared-memory byte address of the top entry of the lane's stack of
-// pending rows.  The entry at `base` is a sentinel: popping an empty stack loads it,
-// and a step leaves the sentinel state {avail 0, nc 1<<31, l 1<<30, r 0} unchanged
-// (no candidate appears and nothing is counted; bit 31 is never a column since
-// n <= 31), so a lane whose search is over parks without a branch.  Entries of a lane
-// sit BLOCK x 16 bytes apart ([level][BLOCK] layout), so the 32 lanes of a warp touch 32
-// consecutive 16-byte slots and an LDS.128 / STS.128 needs no bank replays.
+// pending rows.  Entries of a lane sit BLOCK x 16 bytes apart ([level][BLOCK] layout), so
+// the 32 lanes of a warp touch 32 consecutive 16-byte slots and an LDS.128 / STS.128 needs
+// no bank replays.
 //
 // Per step: if the row has no candidate left, pop the deepest pending row; place the
 // lowest candidate b (avail & (avail - 1) is the row without it, and their XOR is b); push
 // the row back only if candidates remain; step to the next
 // row and "enter" it.  A row left without candidates is not pushed, so a row with one
 // free column is filled without creating a branch point: the reference's unit-row
-// propagation (GPU_NQueens.cu:392-408, n_queens.cuh:145-163).  b is a free column, so it
-// is in nc and in neither diagonal mask, and the updates nc ^= b, l = (l|b) << 1,
-// r = (r|b) >> 1 are written as subtractions and additions, which spreads them over the
-// integer ALU and the IMAD pipe.
+// propagation (GPU_NQueens.cu:392-408, n_queens.cuh:145-163).  The next row's masks are
+// nc & ~b, l + 2b and r' = (r + b) >> 1 (b is a free column, so it is in neither diagonal
+// mask and adding is setting).  Keeping l one row ahead makes its update one multiply-add.
+//
+// The entry at `base` is a sentinel with many candidates and a row whose columns are all
+// attacked.  A lane whose search is over pops it, takes its lowest bit, pushes the rest back
+// into the same slot and enters a row without candidates: nothing is counted, and no
+// instruction guards the stack's bottom.  Each pop uses up one of the sentinel's bits, so the
+// kernels call refresh_sentinel at least every kMaxParkedSteps steps.
 //
 // Entering a row counts every candidate of the row as a node at once: the search places
 // each of them exactly once, so nodes = the sum of the candidate counts of the rows
@@ -30,16 +33,25 @@
 // board (a solution).
 //
 // Dead ends are then counted without being visited.  Placing candidate c leaves the next
-// row with the candidates G & ~{c-1, c, c+1}, where G = nc & ~((l << 1) | (r >> 1)) are the
+// row with the candidates G & ~{c-1, c, c+1}, where G = nc & ~(l | (r >> 1)) are the
 // columns free two rows down from the queens above (c's own column and diagonals aside).
-// So c leads to an empty row -- a leaf, whose node was just counted -- exactly when G lies
-// inside {c-1, c, c+1}.  When G is empty every candidate is a leaf; when G is one column g
-// the leaves are the candidates in {g-1, g, g+1}.  Both cases are removed from `avail`
-// before the row is searched (G of two or three adjacent columns also makes leaves; those
-// are few and are searched normally, which costs a step but counts them the same way).  At
-// N=17..21 this removes 34% of the placements from the step loop and a third of the stack
-// pushes and pops.  The last row is always removed this way, so no step ever places a queen
-// there.
+// So c has a child exactly when G has a column g <= c - 2 or g >= c + 2, that is when c is
+// above lowest(G) + 1 or below highest(G) - 1.  With H = 2G, which needs no right shift
+// (2nc & ~(2l | r)), H ^ -H are the bits above lowest(G) + 1 and 0x1FFFFFFF >> clz(H) those
+// below highest(G) - 1.  All other candidates are
+// leaves, whose nodes were just counted, and are removed from `avail` before the row is
+// searched.  At N=17..21 this removes 36% of the placements from the step loop.  The last
+// row is always removed this way (G is at most its own column), so no step ever places a
+// queen there, and a row entered by a step always has a candidate.
+//
+// What bounds a step: instruction issue and the shared-memory pipe (an LDS.128 and an
+// STS.128, 4 wavefronts each whenever some lane of each 8 takes part) together.  At N=19,
+// depth 7 a warp step issues 28.5 instructions (82% of the issue slots) and keeps the
+// shared-memory pipe 90% busy; with five instructions taken out it runs 8% faster, at 98%
+// of that pipe.  The step before it, with a filter for one-column G only, a compare that
+// guarded the stack's bottom, and shifts where this one has multiply-adds, issued 32.2
+// instructions and made 3.6% more steps: 1/16 of the N=20 depth-7 pool (1.18e11 nodes)
+// took 80.2 ms against 72.0 ms.
 //
 // Stack bound: a row is pushed only while another candidate remains, and pushed rows are
 // strictly deeper towards the top, so a search from a state with f free columns holds at
@@ -56,21 +68,23 @@
 
 namespace nqb {
 
-constexpr uint32_t kSentinelNc = 0x80000000u;
-constexpr uint32_t kSentinelL = 0x40000000u;
+// The sentinel.  Its row has two columns (29 and 30), both attacked there and in the rows
+// after it, which the bits placed one after another (27 of them, all lower) do not change.
+constexpr uint32_t kSentinelAvail = 0x07FFFFFFu, kSentinelNc = 0x60000000u, kSentinelL = 0xF0000000u;
+constexpr int kMaxParkedSteps = 26;  // steps a parked lane may take between refreshes of its sentinel
 
 struct Lane {
     uint32_t avail, nc, l, r;
     uint32_t sp;     // shared byte address of the top entry; == base when the stack is empty
     uint32_t sols;   // solutions since the last fold
     uint32_t nodes;  // placements since the last fold
+    uint32_t placed; // instrumented kernels: steps that placed a queen since the last fold
     uint32_t err;    // NQB_CHECKS builds: bit 0 = a push would have passed the lane's last slot
 };
 
-// What one step did, for the optional counters of the kernels.
+// The candidates of the two rows a pair of steps entered (before dead ends are dropped).
 struct StepInfo {
-    uint32_t placed;  // the column placed (0: the lane is parked)
-    uint32_t cand;    // candidates of the row entered (before dead ends are dropped)
+    uint32_t cand0, cand1;
 };
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -88,107 +102,103 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
 }
 
 __device__ __forceinline__ void write_sentinel(uint32_t addr) {
-    sts128(addr, make_uint4(0u, kSentinelNc, kSentinelL, 0u));
+    sts128(addr, make_uint4(kSentinelAvail, kSentinelNc, kSentinelL, 0u));
 }
 
-// Candidates `a` of a row minus those whose placement leaves the next row empty, when
-// G (see the file comment) has at most one column.  Same arithmetic as the step's.
+// Gives the sentinel all its bits back.  Every lane may do so at any time: the slot at `base`
+// never holds anything else.
+__device__ __forceinline__ void refresh_sentinel(uint32_t base) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(base), "r"(kSentinelAvail) : "memory");
+}
+
+// Candidates `a` of a row minus those whose placement leaves the next row empty (see the
+// file comment); masks as in Lane.  Same arithmetic as the step's.
 __device__ __forceinline__ uint32_t drop_leaves(uint32_t a, uint32_t nc, uint32_t l, uint32_t r) {
-    const uint32_t g = nc & ~((l << 1) | (r >> 1));
-    if ((g & (0u - g)) != g) return a;
-    return g ? a & ~((g * 7u) >> 1) : 0u;
+    const uint32_t h = (nc << 1) & ~((l << 1) | r);
+    return h ? a & ((h ^ (0u - h)) | (0x1FFFFFFFu >> __clz(h))) : 0u;
 }
 
-// PTX of the row entry (candidates, node and solution counts, dead ends dropped), shared
-// by both builds of the step: %0 avail, %1 nc, %2 l, %3 r, %5 nodes, %6 sols, %8 cand.
-#define NQB_ENTER_ROW                                                   \
-    "or.b32 x, %2, %3;\n\t"                                             \
-    "not.b32 x, x;\n\t"                                                 \
-    "and.b32 %0, %1, x;\n\t"         /* candidates of the entered row */ \
-    "popc.b32 %8, %0;\n\t"                                              \
-    "add.u32 %5, %5, %8;\n\t"        /* each is placed once: nodes */    \
-    "sub.u32 x, %1, 1;\n\t"                                             \
-    "and.b32 x, x, %1;\n\t"                                             \
-    "setp.eq.u32 u, x, 0;\n\t"       /* one free column: the last row */ \
-    "@u add.u32 %6, %6, %8;\n\t"     /* its candidate is a solution */   \
-    "shl.b32 g, %2, 1;\n\t"                                             \
-    "shr.u32 x, %3, 1;\n\t"                                             \
-    "or.b32 g, g, x;\n\t"                                               \
-    "not.b32 g, g;\n\t"                                                 \
-    "and.b32 g, g, %1;\n\t"          /* G */                             \
-    "neg.s32 x, g;\n\t"                                                 \
-    "not.b32 w, x;\n\t"                                                 \
-    "and.b32 w, w, g;\n\t"                                              \
-    "setp.eq.u32 u, w, 0;\n\t"       /* G has at most one column */      \
-    "shr.s32 x, x, 31;\n\t"          /* all ones iff G != 0 */           \
-    "mul.lo.u32 w, g, 7;\n\t"                                           \
-    "shr.u32 w, w, 1;\n\t"           /* {g-1, g, g+1} */                 \
-    "not.b32 w, w;\n\t"                                                 \
-    "and.b32 w, w, x;\n\t"                                              \
-    "@u and.b32 %0, %0, w;\n\t"      /* drop the leaves */
+// PTX of one step from the registers {a, n, l, r} into {A, N, L, R}: the previous and the next
+// step's avail, nc, l, r.  `push` is the push of the quad {a, n, l, r}; c receives the
+// candidates of the row entered.
+#define NQB_STEP(a, n, l, r, A, N, L, R, c, push, count)                                                 \
+    "setp.eq.u32 p, " a ", 0;\n\t" /* no candidate left: pop */                                          \
+    count                                                                                                \
+    "@p ld.shared.v4.u32 {" a ", " n ", " l ", " r "}, [%4];\n\t"                                        \
+    "@p sub.u32 %4, %4, %10;\n\t"                                                                        \
+    "sub.u32 x, " a ", 1;\n\t"                                                                           \
+    "not.b32 w, x;\n\t"                                                                                  \
+    "and.b32 b, " a ", w;\n\t"     /* the row's lowest candidate b */                                    \
+    "and.b32 " a ", " a ", x;\n\t" /* the row without it */                                              \
+    "setp.ne.u32 t, " a ", 0;\n\t" /* candidates remain: push the row */                                 \
+    push                                                                                                 \
+    "not.b32 x, b;\n\t"                                                                                  \
+    "and.b32 " N ", " n ", x;\n\t"                                                                       \
+    "mad.lo.u32 x, b, 2, " l ";\n\t"                                                                     \
+    "shl.b32 " L ", x, 1;\n\t"                                                                           \
+    "shl.b32 h, x, 2;\n\t"                                                                               \
+    "add.u32 w, " r ", b;\n\t"                                                                           \
+    "shr.u32 " R ", w, 1;\n\t"                                                                           \
+    "or.b32 w, x, " R ";\n\t"                                                                            \
+    "not.b32 w, w;\n\t"                                                                                  \
+    "and.b32 " A ", " N ", w;\n\t" /* candidates of the entered row */                                   \
+    "popc.b32 " c ", " A ";\n\t"                                                                         \
+    "sub.u32 w, " N ", 1;\n\t"                                                                           \
+    "and.b32 w, w, " N ";\n\t"                                                                           \
+    "setp.eq.u32 u, w, 0;\n\t"        /* one free column: the last row */                                \
+    "@u add.u32 %5, %5, " c ";\n\t"   /* its candidate is a solution */                                  \
+    "shl.b32 x, " N ", 1;\n\t"                                                                           \
+    "or.b32 w, h, " R ";\n\t"                                                                            \
+    "not.b32 w, w;\n\t"                                                                                  \
+    "and.b32 h, x, w;\n\t"            /* H */                                                            \
+    "neg.s32 w, h;\n\t"                                                                                  \
+    "xor.b32 w, w, h;\n\t"            /* above lowest(G) + 1 */                                          \
+    "bfind.shiftamt.u32 x, h;\n\t"    /* clz(H), all ones for H = 0 */                                   \
+    "shr.u32 x, k, x;\n\t"            /* below highest(G) - 1 */                                         \
+    "or.b32 w, w, x;\n\t"                                                                                \
+    "and.b32 " A ", " A ", w;\n\t"    /* drop the leaves */
 
-// One step; STRIDE is the byte distance between a lane's stack entries (BLOCK x 16);
-// `top` is the byte address of the lane's last stack slot (checked builds only).
-template <int STRIDE>
-__device__ __forceinline__ StepInfo search_step(Lane& s, uint32_t base, uint32_t top) {
-    StepInfo o;
 #ifndef NQB_CHECKS
-    (void)top;
-    asm volatile(
-        "{\n\t.reg .pred p, q, t, u;\n\t.reg .u32 x, g, w;\n\t"
-        "setp.eq.u32 p, %0, 0;\n\t"                        // no candidate left: pop
-        "@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
-        "setp.ne.and.u32 q, %4, %9, p;\n\t"
-        "@q sub.u32 %4, %4, %10;\n\t"
-        "sub.u32 x, %0, 1;\n\t"                            // the row without its lowest candidate b
-        "and.b32 x, x, %0;\n\t"
-        "setp.ne.u32 t, x, 0;\n\t"                         // candidates remain: push the row
-        "xor.b32 %7, %0, x;\n\t"
-        "mov.u32 %0, x;\n\t"
-        "@t add.u32 %4, %4, %10;\n\t"
-        "@t st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"
-        "sub.u32 %1, %1, %7;\n\t"                          // next row
-        "add.u32 %2, %2, %7;\n\t"
-        "shl.b32 %2, %2, 1;\n\t"
-        "add.u32 %3, %3, %7;\n\t"
-        "shr.u32 %3, %3, 1;\n\t"
-        NQB_ENTER_ROW
-        "}"
-        : "+r"(s.avail), "+r"(s.nc), "+r"(s.l), "+r"(s.r), "+r"(s.sp), "+r"(s.nodes), "+r"(s.sols),
-          "=r"(o.placed), "=r"(o.cand)
-        : "r"(base), "n"(STRIDE)
-        : "memory");
+#define NQB_PUSH(a, n, l, r)       \
+    "@t add.u32 %4, %4, %10;\n\t" \
+    "@t st.shared.v4.u32 [%4], {" a ", " n ", " l ", " r "};\n\t"
 #else
-    asm volatile(
-        "{\n\t.reg .pred p, q, t, u, ov, ok;\n\t.reg .u32 x, g, w, nsp;\n\t"
-        "setp.eq.u32 p, %0, 0;\n\t"
-        "@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
-        "setp.ne.and.u32 q, %4, %10, p;\n\t"
-        "@q sub.u32 %4, %4, %11;\n\t"
-        "sub.u32 x, %0, 1;\n\t"
-        "and.b32 x, x, %0;\n\t"
-        "setp.ne.u32 t, x, 0;\n\t"
-        "xor.b32 %7, %0, x;\n\t"
-        "mov.u32 %0, x;\n\t"
-        "add.u32 nsp, %4, %11;\n\t"                        // the push's slot must not pass top
-        "setp.gt.u32 ov, nsp, %12;\n\t"
-        "and.pred ok, t, !ov;\n\t"
-        "@ok mov.u32 %4, nsp;\n\t"
-        "@ok st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"
-        "and.pred ov, t, ov;\n\t"
-        "@ov or.b32 %9, %9, 1;\n\t"
-        "sub.u32 %1, %1, %7;\n\t"
-        "add.u32 %2, %2, %7;\n\t"
-        "shl.b32 %2, %2, 1;\n\t"
-        "add.u32 %3, %3, %7;\n\t"
-        "shr.u32 %3, %3, 1;\n\t"
-        NQB_ENTER_ROW
-        "}"
-        : "+r"(s.avail), "+r"(s.nc), "+r"(s.l), "+r"(s.r), "+r"(s.sp), "+r"(s.nodes), "+r"(s.sols),
-          "=r"(o.placed), "=r"(o.cand), "+r"(s.err)
-        : "r"(base), "n"(STRIDE), "r"(top)
-        : "memory");
+#define NQB_PUSH(a, n, l, r)                                          \
+    "add.u32 x, %4, %10;\n\t" /* the push's slot must not pass top */ \
+    "setp.gt.u32 ov, x, %12;\n\t"                                     \
+    "and.pred ok, t, !ov;\n\t"                                        \
+    "@ok mov.u32 %4, x;\n\t"                                          \
+    "@ok st.shared.v4.u32 [%4], {" a ", " n ", " l ", " r "};\n\t"    \
+    "and.pred ov, t, ov;\n\t"                                         \
+    "@ov or.b32 %8, %8, 1;\n\t"
 #endif
+
+// Counts a step that places a queen: one that does not pop the sentinel.
+#define NQB_COUNT_PLACED                 \
+    "setp.ne.or.u32 q, %4, %11, !p;\n\t" \
+    "@q add.u32 %9, %9, 1;\n\t"
+
+#define NQB_TWO_STEPS(count)                                                                                    \
+    asm volatile(                                                                                               \
+        "{\n\t.reg .pred p, q, t, u, ov, ok;\n\t.reg .u32 b, x, h, w, k, a1, n1, l1, r1;\n\t"                   \
+        "mov.u32 k, 0x1FFFFFFF;\n\t"                                                                            \
+        NQB_STEP("%0", "%1", "%2", "%3", "a1", "n1", "l1", "r1", "%6", NQB_PUSH("%0", "%1", "%2", "%3"), count) \
+        NQB_STEP("a1", "n1", "l1", "r1", "%0", "%1", "%2", "%3", "%7", NQB_PUSH("a1", "n1", "l1", "r1"), count) \
+        "}"                                                                                                     \
+        : "+r"(s.avail), "+r"(s.nc), "+r"(s.l), "+r"(s.r), "+r"(s.sp), "+r"(s.sols), "=&r"(o.cand0),            \
+          "=&r"(o.cand1), "+r"(s.err), "+r"(s.placed)                                                           \
+        : "n"(STRIDE), "r"(base), "r"(top)                                                                      \
+        : "memory")
+
+// Two steps (their candidate counts then join the node count in one addition); STRIDE is the byte distance between a lane's stack entries (BLOCK x 16); `top` is
+// the byte address of the lane's last stack slot (checked builds only); LANES: s.placed counts
+// the steps that place a queen.
+template <int STRIDE, bool LANES>
+__device__ __forceinline__ StepInfo search_two_steps(Lane& s, uint32_t base, uint32_t top) {
+    StepInfo o;
+    if (LANES) NQB_TWO_STEPS(NQB_COUNT_PLACED);
+    else NQB_TWO_STEPS("");
+    s.nodes += o.cand0 + o.cand1;  // each candidate is placed once: nodes
     return o;
 }
 
@@ -199,10 +209,10 @@ __device__ __forceinline__ uint32_t lane_load(Lane& s, const uint4 st, uint32_t 
     const uint32_t n = (st.w >> 8) & 0xFFu;
     const uint32_t mask = n >= 32 ? 0xFFFFFFFFu : ((1u << n) - 1u);
     s.nc = mask & ~st.x;
-    s.l = st.y;
+    s.l = st.y << 1;
     s.r = st.z;
     s.sp = base;
-    const uint32_t a = s.nc & ~(s.l | s.r);
+    const uint32_t a = s.nc & ~(st.y | st.z);
     const uint32_t pc = __popc(a);
     s.nodes = pc;
     s.sols = (s.nc & (s.nc - 1u)) == 0 ? pc + (s.nc == 0) : 0u;
@@ -214,9 +224,7 @@ __device__ __forceinline__ uint32_t lane_load(Lane& s, const uint4 st, uint32_t 
 // Empties a lane: the next step pops the sentinel.
 __device__ __forceinline__ void lane_park(Lane& s, uint32_t base) {
     s.avail = 0;
-    s.nc = kSentinelNc;
-    s.l = kSentinelL;
-    s.r = 0;
+    s.nc = s.l = s.r = 0;
     s.sp = base;
 }
 
