@@ -81,6 +81,23 @@ int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d
                    unsigned stack_depth, int device, cudaStream_t stream, unsigned* launches,
                    unsigned long long* d_lane_stats = nullptr, uint32_t wait_limit = 0);
 
+// Items split until a launch has several a lane (refine.cu): the caller's arrays, or device
+// copies owned until release() (a stream-ordered free).  Placements of split items are added
+// into d_totals[1] (unit: the unit ones also into d_totals[2]) and d_board_nodes[board].
+// boards: the items' output slots are needed.  Waits for the stream when it splits.
+struct Refined {
+    const nqb_state* items = nullptr;
+    const uint32_t* board = nullptr;  // item -> output slot (nullptr: identity)
+    uint32_t n = 0;
+    unsigned stack_depth = 0;         // bound of the items as they are now
+    void* buf = nullptr;
+    cudaStream_t stream = nullptr;
+    void release();
+};
+int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, bool boards, bool unit,
+                 unsigned stack_depth, int device, cudaStream_t s, unsigned long long* d_totals,
+                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out);
+
 // Items after learned scheduling: the caller's arrays, or split / ordered device copies
 // owned by the schedule until release() (stream-ordered frees).
 struct Schedule {
@@ -103,7 +120,8 @@ int schedule_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board
                    Schedule* out);
 
 // Batched form with optional learned scheduling (schedule.cu): with o.model, items are
-// split and ordered by predicted cost before the launch; otherwise launched as given.
+// split and ordered by predicted cost before the launch; otherwise few items are split
+// (refine.cu) and the queue keeps no order.
 struct SchedInfo {
     uint64_t items = 0;     // items given to the search kernel
     double sched_ms = 0.0;  // prediction + splitting + ordering (device time)

@@ -1,0 +1,219 @@
+// Splits the items of a launch that has too few of them.
+//
+// A search kernel keeps its lanes busy only while it has several items a lane: with fewer,
+// the time goes into handing pieces of long subtrees from lane to lane and from warp to warp.
+// Before such a launch the items are split into their children, level by level, until there
+// are kItemsPerLane a lane: a device pass over a few hundred thousand 16-byte items against a
+// search of milliseconds.
+//
+// One level: an item with many free columns is replaced by its children, one per candidate
+// of its next row that has a child itself (the step's leaf filter, search_step.cuh); the
+// candidates are counted as nodes here, and the children are searched like any other item, so
+// counts, nodes and unit nodes are those of the unsplit search.  Only items within
+// kSplitSpread free columns of the largest are split, so the small boards of an uneven batch
+// stay whole.  Children are appended behind an atomic count, one reservation a warp, so a level
+// needs neither a scan nor a read-back; the order of the items is not kept (no result depends
+// on it).  While a level writes its items it adds up how many the next level would make, so
+// each level knows before it starts whether it fits the buffers, and hands its input on
+// unchanged when it does not, when nothing would be split or when there are items enough.
+//
+// What bounds it: launch latency (a level is a few microseconds).  Batched form, whole calls:
+// N=18 at pool depths 3 and 4 (1,710 and 18,132 items, split to 1.2M) 33.4 -> 19.0 ms, the time
+// of the depth-6 pool; 8,192 uneven boards (n 16-20, split to 2.1M) 244 -> 215 ms.  With two
+// items a lane the queue's tail is a few percent; four a lane were no faster.
+#include <algorithm>
+
+#include "nqb_internal.h"
+#include "search_step.cuh"
+
+namespace nqb {
+namespace {
+
+constexpr unsigned kFull = 0xFFFFFFFFu;
+constexpr uint32_t kItemsPerLane = 2;      // levels stop at this many items a resident lane
+constexpr uint32_t kCapItems = 3200000;    // room of each of the two buffers (51 MB)
+constexpr uint32_t kMinSplitFree = 8;      // items with fewer free columns are a few hundred nodes
+constexpr uint32_t kSplitSpread = 3;
+constexpr unsigned kMaxLevels = 4;
+constexpr unsigned kThreads = 256;
+
+struct Level {
+    const uint4* items;
+    const uint32_t* board;      // item -> output slot (nullptr: identity)
+    unsigned long long next;    // items the next level would make of these
+    uint32_t n;
+    uint32_t done;              // levels that split something
+};
+
+__device__ __forceinline__ uint32_t free_columns(const uint4 s) {
+    const uint32_t n = (s.w >> 8) & 0xFFu;
+    return (n >= 32 ? 0xFFFFFFFFu : ((1u << n) - 1u)) & ~s.x;
+}
+
+// The candidates of an item's next row that have a child.
+__device__ __forceinline__ uint32_t living(const uint4 s, uint32_t nc) {
+    return drop_leaves(nc & ~(s.y | s.z), nc, s.y << 1, s.z);
+}
+
+// Items that `s` becomes in a level that splits from `cut` free columns on.
+__device__ __forceinline__ uint32_t made_of(const uint4 s, uint32_t cut) {
+    const uint32_t nc = free_columns(s);
+    return (uint32_t)__popc(nc) >= cut ? __popc(living(s, nc)) : 1u;
+}
+
+__global__ void first_kernel(const uint4* __restrict__ items, const uint32_t* __restrict__ board, uint32_t n,
+                             uint32_t cut, Level* __restrict__ out) {
+    unsigned long long made = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        made += made_of(__ldg(items + i), cut);
+    made = warp_sum_u64(made);
+    if ((threadIdx.x & 31) == 0 && made) atomicAdd(&out->next, made);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out->items = items;
+        out->board = board;
+        out->n = n;
+    }
+}
+
+// One level: in -> out, or `in` handed on.  UNIT: children whose row has exactly one candidate
+// are counted as unit placements (a search kernel takes an item's first row for a start row).
+template <bool UNIT>
+__global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict__ in, Level* __restrict__ out,
+                                                         uint4* __restrict__ to, uint32_t* __restrict__ to_board,
+                                                         uint32_t cut, uint32_t next_cut, uint32_t enough,
+                                                         unsigned long long* __restrict__ totals,
+                                                         unsigned long long* __restrict__ board_nodes) {
+    const uint32_t n = in->n;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (n >= enough || in->next > kCapItems || in->next == n) {
+        if (first) {
+            out->items = in->items;
+            out->board = in->board;
+            out->n = n;
+            out->next = n;  // the levels after this one hand it on too
+            out->done = in->done;
+        }
+        return;
+    }
+    const uint4* const items = in->items;
+    const uint32_t* const board = in->board;
+    const uint32_t lane = threadIdx.x & 31;
+    unsigned long long nodes = 0, made = 0;
+    uint32_t units = 0;
+    for (uint32_t i0 = (blockIdx.x * kThreads + threadIdx.x) & ~31u; i0 < n; i0 += gridDim.x * kThreads) {
+        const uint32_t i = i0 + lane;
+        const bool valid = i < n;
+        const uint4 s = valid ? items[i] : make_uint4(0, 0, 0, 0);
+        const uint32_t id = valid && to_board ? (board ? board[i] : i) : 0u;
+        const uint32_t nc = free_columns(s);
+        const bool split = valid && (uint32_t)__popc(nc) >= cut;
+        const uint32_t kids = split ? living(s, nc) : 0u;
+        if (split) {
+            const uint32_t placed = __popc(nc & ~(s.y | s.z));
+            nodes += placed;
+            if (board_nodes && placed) atomicAdd(board_nodes + id, (unsigned long long)placed);
+        }
+        const uint32_t c = split ? __popc(kids) : (uint32_t)valid;
+        uint32_t p = c;  // inclusive prefix over the warp
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, p, d);
+            if (lane >= (uint32_t)d) p += v;
+        }
+        const uint32_t total = __shfl_sync(kFull, p, 31);
+        p -= c;
+        uint32_t at = 0;
+        if (lane == 0 && total) at = atomicAdd(&out->n, total);
+        at = __shfl_sync(kFull, at, 0) + p;
+        // total <= what `in` promised, so at + c stays inside the buffer
+        uint32_t left = kids;
+        for (uint32_t j = 0; j < c; ++j) {
+            uint4 o = s;
+            if (split) {
+                const uint32_t b = left & (0u - left);
+                left ^= b;
+                o = make_uint4(s.x | b, (s.y | b) << 1, (s.z | b) >> 1, s.w);  // no kernel reads the row number
+                if (UNIT) units += __popc(free_columns(o) & ~(o.y | o.z)) == 1;
+            }
+            to[at + j] = o;
+            if (to_board) to_board[at + j] = id;
+            made += made_of(o, next_cut);
+        }
+    }
+    nodes = warp_sum_u64(nodes);
+    made = warp_sum_u64(made);
+    unsigned long long unit64 = units;
+    if (UNIT) unit64 = warp_sum_u64(unit64);
+    if (lane == 0) {
+        if (nodes) atomicAdd(totals + 1, nodes);
+        if (UNIT && unit64) atomicAdd(totals + 2, unit64);
+        if (made) atomicAdd(&out->next, made);
+    }
+    if (first) {
+        out->items = to;
+        out->board = to_board;
+        out->done = in->done + 1;
+    }
+}
+
+}  // namespace
+
+void Refined::release() {
+    if (buf) dev_free(buf, stream);
+    buf = nullptr;
+}
+
+int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, bool boards, bool unit,
+                 unsigned stack_depth, int device, cudaStream_t s, unsigned long long* d_totals,
+                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out) {
+    out->items = d_items;
+    out->board = d_board;
+    out->n = n;
+    out->stack_depth = stack_depth;
+    int sms = 0;
+    NQB_TRY(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)));
+    const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;  // 36 warps of an SM's stack memory
+    const uint32_t max_free = stack_depth + 1;
+    if (n >= enough || max_free <= kMinSplitFree) return NQB_OK;
+    const unsigned levels = std::min(kMaxLevels, max_free - kMinSplitFree);
+    auto cut_of = [&](unsigned level) {  // free columns from which a level splits
+        const uint32_t top = max_free - level;
+        return std::max(kMinSplitFree, top > kSplitSpread ? top - kSplitSpread : 0u);
+    };
+    boards = boards || d_board;
+    const size_t item_bytes = (size_t)kCapItems * sizeof(uint4);
+    const size_t board_bytes = boards ? (size_t)kCapItems * sizeof(uint32_t) : 0;
+    const size_t head = (kMaxLevels + 1) * sizeof(Level) + 64;
+    void* mem = nullptr;
+    NQB_TRY(dev_alloc_bytes(&mem, 512 + 2 * (item_bytes + board_bytes), s));
+    static_assert((kMaxLevels + 1) * sizeof(Level) + 64 <= 512, "the level records have 512 bytes");
+    out->buf = mem;
+    out->stream = s;
+    char* const base = static_cast<char*>(mem);
+    Level* const lv = reinterpret_cast<Level*>(base);
+    NQB_TRY(cuda_status(cudaMemsetAsync(lv, 0, head, s)));
+    const unsigned grid0 = std::max(1u, std::min((n + kThreads - 1) / kThreads, 4u * (unsigned)sms));
+    first_kernel<<<grid0, kThreads, 0, s>>>(reinterpret_cast<const uint4*>(d_items), d_board, n, cut_of(0), lv);
+    for (unsigned k = 0; k < levels; ++k) {
+        char* const to = base + 512 + (k & 1) * (item_bytes + board_bytes);
+        uint4* const to_items = reinterpret_cast<uint4*>(to);
+        uint32_t* const to_board = boards ? reinterpret_cast<uint32_t*>(to + item_bytes) : nullptr;
+        auto kern = unit ? level_kernel<true> : level_kernel<false>;
+        kern<<<4 * sms, kThreads, 0, s>>>(lv + k, lv + k + 1, to_items, to_board, cut_of(k), cut_of(k + 1), enough,
+                                          d_totals, d_board_nodes);
+    }
+    NQB_TRY(cuda_status(cudaGetLastError()));
+    if (launches) *launches += 1 + levels;
+    Level last;
+    NQB_TRY(cuda_status(cudaMemcpyAsync(&last, lv + levels, sizeof(last), cudaMemcpyDeviceToHost, s)));
+    NQB_TRY(cuda_status(cudaStreamSynchronize(s)));
+    out->items = reinterpret_cast<const nqb_state*>(last.items);
+    out->board = last.board;
+    out->n = last.n;
+    // Every item with more than max_free - done free columns has been split (a level's cut is
+    // at most its largest), unless the cut was held at kMinSplitFree.
+    out->stack_depth = std::max(stack_depth > last.done ? stack_depth - last.done : 1u, 1u);
+    return NQB_OK;
+}
+
+}  // namespace nqb

@@ -13,7 +13,8 @@
 //      to max_split_rounds rounds or until nothing is split;
 //   3. order the queue by predicted cost, largest first (CUB radix sort of (cost, index));
 //   4. one launch of the batched kernel with that order.
-// Without a model the items go to the kernel unchanged, in their given order (FIFO), unless
+// Without a model the items go to the kernel in no particular order, few items split first
+// (refine.cu), unless
 // a model-free cost is asked for (nqb_opts.sched_cost: the ablation arms of the learned
 // schedule), which then drives the same split-and-order steps in place of the prediction.
 #include <algorithm>
@@ -261,6 +262,17 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
                              unsigned long long* d_per_board_nodes, const nqb_opts& o, unsigned stack_depth,
                              int device, cudaStream_t s, unsigned* launches, SchedInfo* info,
                              unsigned long long* d_lane_stats) {
+    if (!o.model && o.sched_cost == 0) {
+        Refined r;
+        int st = refine_items(d_items, n, d_board, d_per_board || d_per_board_nodes, false, stack_depth, device, s,
+                              d_out, d_per_board_nodes, launches, &r);
+        if (!st)
+            st = launch_batched(r.items, r.n, nullptr, r.board, d_scratch, scratch_bytes, d_out, d_per_board,
+                                d_per_board_nodes, o.block_size, r.stack_depth, device, s, launches, d_lane_stats);
+        r.release();  // stream-ordered after the kernel that reads the arrays
+        if (info) info->items = r.n;
+        return st;
+    }
     Schedule sch;
     int st = schedule_items(d_items, n, d_board, o, device, s, d_out + 1, d_per_board_nodes, &sch);
     if (!st)

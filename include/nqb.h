@@ -113,7 +113,7 @@ typedef struct nqb_stats {
     double wall_ms;      /* whole call                                             */
     uint32_t pregen_depth;
     uint32_t kernel_launches;
-    uint64_t items;      /* items the search kernel was given (after learned splitting) */
+    uint64_t items;      /* items the search kernel was given (after any splitting)      */
     double sched_ms;     /* learned scheduling: prediction, splitting, ordering        */
     uint32_t block_size; /* threads per block of the search launch                        */
     int32_t form;        /* search form used (NQB_FORM_*)                                  */
