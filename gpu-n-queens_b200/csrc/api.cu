@@ -132,8 +132,8 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
                                              d_per, d_per_nodes, o, depth, sc.device, sc.stream, &launches, &sched,
                                              d_lanes));
         } else {
-            NQB_TRY(launch_plain(d_states, count, d_out, d_per, o.block_size, o.count_unit_nodes != 0, depth,
-                                 sc.stream, &launches, d_lanes));
+            NQB_TRY(launch_plain_refined(d_states, count, d_out, d_per, o, depth, sc.device, sc.stream, &launches,
+                                         &sched, d_lanes));
         }
     }
     NQB_TRY(cuda_status(cudaEventRecord(e2, sc.stream)));

@@ -282,38 +282,7 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
                         rounds = 0;
                     }
                 } else {
-                    const uint32_t k = min(__popc(idle), __popc(donors));
-                    const uint32_t ri = __popc(idle & lt_mask);    // rank among idle lanes
-                    const uint32_t rd = __popc(donors & lt_mask);  // rank among donors
-                    const bool recv = me_idle && ri < k;
-                    const bool give = ((donors >> lane) & 1u) && rd < k;
-                    uint32_t src = lane;
-                    if (recv) {  // lane of the ri-th donor
-                        uint32_t m = donors;
-                        for (uint32_t j = 0; j < ri; ++j) m &= m - 1u;
-                        src = __ffs(m) - 1;
-                    }
-                    const uint32_t slot = __shfl_sync(kFull, base + kStride, src);  // donor's bottom row
-                    const uint32_t dw = __shfl_sync(kFull, weight, src);
-                    const uint32_t ditem = __shfl_sync(kFull, item, src);
-                    __syncwarp();
-                    if (recv) {
-                        const uint4 e = lds128(slot);
-                        base = base0;
-                        write_sentinel(base0);
-                        s.avail = e.x;
-                        s.nc = e.y;
-                        s.l = e.z;
-                        s.r = e.w;
-                        s.sp = base;
-                        weight = dw;
-                        item = ditem;
-                    }
-                    __syncwarp();
-                    if (give) {  // the handed-over row's slot becomes the new sentinel
-                        base += kStride;
-                        write_sentinel(base);
-                    }
+                    share_rows<kStride>(s, base, base0, weight, item, idle, donors, lane);
                 }
             }
         }

@@ -53,11 +53,13 @@ unsigned host_threads();
 unsigned max_stack_depth(const nqb_state* states, uint64_t count);
 
 // Plain search kernel (plain.cu).  d_out: {weighted count, nodes, unit nodes, error flags}.
-// d_per_state (optional): weight x completions per state.  d_lane_stats (optional): the
+// d_per_state (optional, zero at launch): weight x completions per state.  d_lane_stats (optional): the
 // instrumented kernel adds {lane-steps that placed a queen, lane-step slots} into it.
+// d_board_of (optional): state -> slot of d_per_state.
 int launch_plain(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
                  unsigned long long* d_per_state, int block_size, bool count_unit, unsigned stack_depth,
-                 cudaStream_t stream, unsigned* launches, unsigned long long* d_lane_stats = nullptr);
+                 cudaStream_t stream, unsigned* launches, unsigned long long* d_lane_stats = nullptr,
+                 const uint32_t* d_board_of = nullptr);
 
 // Scratch of one batched launch (zeroed before it): 64 bytes of control words (word 0 is
 // the item queue head), then the steal ring, 32 bytes a slot.  Scratch of 4 bytes (the
@@ -131,6 +133,12 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
                              unsigned long long* d_per_board_nodes, const nqb_opts& o, unsigned stack_depth,
                              int device, cudaStream_t s, unsigned* launches, SchedInfo* info,
                              unsigned long long* d_lane_stats = nullptr);
+
+// Plain form of the library's own calls: few items are split first (refine.cu).
+int launch_plain_refined(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
+                         unsigned long long* d_per_state, const nqb_opts& o, unsigned stack_depth, int device,
+                         cudaStream_t s, unsigned* launches, SchedInfo* info,
+                         unsigned long long* d_lane_stats = nullptr);
 
 // Stream-ordered device allocation from the library's pool on the current device
 // (devmem.cu); release with dev_free on a stream.  Freed memory stays cached for later

@@ -19,8 +19,9 @@
 //
 // What bounds it: launch latency (a level is a few microseconds).  Batched form, whole calls:
 // N=18 at pool depths 3 and 4 (1,710 and 18,132 items, split to 1.2M) 33.4 -> 19.0 ms, the time
-// of the depth-6 pool; 8,192 uneven boards (n 16-20, split to 2.1M) 244 -> 215 ms.  With two
-// items a lane the queue's tail is a few percent; four a lane were no faster.
+// of the depth-6 pool; 8,192 uneven boards (n 16-20, split to 2.1M) 244 -> 215 ms.  Stopping
+// at one item a lane leaves N=19 at depth 4 at 165 ms and the uneven boards at 239 ms, against
+// 147.5 and 209 ms (same box) at two; at four, calls move within 4% either way.
 #include <algorithm>
 
 #include "nqb_internal.h"

@@ -287,4 +287,22 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
     return st;
 }
 
+int launch_plain_refined(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
+                         unsigned long long* d_per_state, const nqb_opts& o, unsigned stack_depth, int device,
+                         cudaStream_t s, unsigned* launches, SchedInfo* info, unsigned long long* d_lane_stats) {
+    const bool unit = o.count_unit_nodes != 0;
+    if (count > 0xFFFFFFFFull)  // far more than the split is for
+        return launch_plain(d_states, count, d_out, d_per_state, o.block_size, unit, stack_depth, s, launches,
+                            d_lane_stats);
+    Refined r;
+    int st = refine_items(d_states, (uint32_t)count, nullptr, d_per_state != nullptr, unit, stack_depth, device, s,
+                          d_out, nullptr, launches, &r);
+    if (!st)
+        st = launch_plain(r.items, r.n, d_out, d_per_state, o.block_size, unit, r.stack_depth, s, launches,
+                          d_lane_stats, r.board);
+    r.release();
+    if (info) info->items = r.n;
+    return st;
+}
+
 }  // namespace nqb

@@ -228,6 +228,50 @@ __device__ __forceinline__ void lane_park(Lane& s, uint32_t base) {
     s.sp = base;
 }
 
+// Re-splits work inside a warp: lanes with pending rows (`donors`) hand their shallowest one,
+// the largest piece of what they have left, to the warp's idle lanes.  The receiver searches it
+// as a new piece of the donor's item, from the bottom of its own stack (`base0`); the
+// handed-over row's slot becomes the donor's sentinel, so its `base` moves up one slot.  All
+// 32 lanes call it; `idle` and `donors` are their ballots.
+template <int STRIDE>
+__device__ __forceinline__ void share_rows(Lane& s, uint32_t& base, uint32_t base0, uint32_t& weight, uint32_t& item,
+                                           uint32_t idle, uint32_t donors, uint32_t lane) {
+    constexpr unsigned kAll = 0xFFFFFFFFu;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t k = min(__popc(idle), __popc(donors));
+    const uint32_t ri = __popc(idle & lt_mask);    // rank among idle lanes
+    const uint32_t rd = __popc(donors & lt_mask);  // rank among donors
+    const bool recv = ((idle >> lane) & 1u) && ri < k;
+    const bool give = ((donors >> lane) & 1u) && rd < k;
+    uint32_t src = lane;
+    if (recv) {  // lane of the ri-th donor
+        uint32_t m = donors;
+        for (uint32_t j = 0; j < ri; ++j) m &= m - 1u;
+        src = __ffs(m) - 1;
+    }
+    const uint32_t slot = __shfl_sync(kAll, base + STRIDE, src);  // donor's bottom row
+    const uint32_t dw = __shfl_sync(kAll, weight, src);
+    const uint32_t ditem = __shfl_sync(kAll, item, src);
+    __syncwarp();
+    if (recv) {
+        const uint4 e = lds128(slot);
+        base = base0;
+        write_sentinel(base0);
+        s.avail = e.x;
+        s.nc = e.y;
+        s.l = e.z;
+        s.r = e.w;
+        s.sp = base;
+        weight = dw;
+        item = ditem;
+    }
+    __syncwarp();
+    if (give) {
+        base += STRIDE;
+        write_sentinel(base);
+    }
+}
+
 __device__ __forceinline__ unsigned warp_or(unsigned v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v |= __shfl_down_sync(0xFFFFFFFFu, v, o);

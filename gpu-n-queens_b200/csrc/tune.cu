@@ -45,7 +45,8 @@ int time_candidate(const nqb_state* d_sample, uint32_t count, unsigned depth, co
                 st = launch_batched_scheduled(d_sample, count, nullptr, d_out + 8, kBatchedScratchBytes, d_out,
                                               nullptr, nullptr, o, depth, device, s, &launches, &info);
             } else {
-                st = launch_plain(d_sample, count, d_out, nullptr, c.block, false, depth, s, &launches);
+                SchedInfo info;
+                st = launch_plain_refined(d_sample, count, d_out, nullptr, o, depth, device, s, &launches, &info);
             }
         }
         if (!st) st = cuda_status(cudaEventRecord(e1, s));

@@ -71,7 +71,7 @@ typedef struct nqb_state {
 } nqb_state;
 
 /* ---- options and statistics ------------------------------------------- */
-#define NQB_FORM_PLAIN 0   /* one thread per state, static assignment            */
+#define NQB_FORM_PLAIN 0   /* one thread per state; a warp shares its lanes' work  */
 #define NQB_FORM_BATCHED 1 /* persistent kernel, device work queue, re-splitting */
 
 struct nqb_model; /* learned cost model, see nqb_model_create */
@@ -382,7 +382,8 @@ int nqb_solve_ref_states(unsigned n, const void* ref_states, uint64_t count, uns
 
 /* ---- device-resident launches (inputs already in HBM) ------------------- */
 /*
- * Plain form on states already in device memory: one thread per state.
+ * Plain form on states already in device memory: one thread per state; lanes that are
+ * done take pending rows over from the other lanes of their warp.
  * d_out points to 4 device uint64 words {weighted count, nodes, unit nodes, error
  * flags}; the kernel adds into them, so zero them first.  Unit nodes are counted
  * only with count_unit_nodes != 0.  stack_depth bounds the pending rows one search
