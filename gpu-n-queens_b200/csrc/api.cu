@@ -46,13 +46,12 @@ class Scope {
         status = nqb_device_check(dev);
         if (status != NQB_OK) return;
         if ((status = cuda_status(cudaSetDevice(dev))) != NQB_OK) return;
-        status = cuda_status(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        status = stream_take(&stream);
     }
     ~Scope() {
         for (void* p : bufs_) dev_free(p, stream);
-        if (stream) cudaStreamSynchronize(stream);
+        if (stream) stream_give(stream);
         for (cudaEvent_t e : events_) cudaEventDestroy(e);
-        if (stream) cudaStreamDestroy(stream);
         cudaSetDevice(prev_);
     }
     // The slot is added before the buffer or event is made: a push_back that throws then

@@ -543,7 +543,12 @@ struct Work {
           *loss = nullptr;
     unsigned* err = nullptr;  // set by a GEMM whose tensor-core completion wait timed out
     uint32_t cap = 0;
+    cudaStream_t stream;  // the buffers are allocated and freed in its order
     std::vector<void*> owned;
+
+    explicit Work(cudaStream_t s) : stream(s) {}
+    Work(const Work&) = delete;
+    Work& operator=(const Work&) = delete;
 
     int init(uint32_t rows) {
         cap = rows;
@@ -551,7 +556,7 @@ struct Work {
         owned.reserve(16);  // may throw, but before anything is allocated; push_back then does not
         auto get = [&](auto** p, size_t bytes) {
             void* v = nullptr;
-            const int s = cuda_malloc(&v, bytes);
+            const int s = dev_alloc_bytes(&v, bytes, stream);
             if (s == NQB_OK) {
                 owned.push_back(v);
                 *p = static_cast<std::remove_pointer_t<decltype(p)>>(v);
@@ -573,7 +578,7 @@ struct Work {
         if (!s) s = get(&dH1, r * kH * sizeof(float));
         if (!s) s = get(&loss, sizeof(float));
         if (!s) s = get(&err, sizeof(unsigned));
-        if (!s) s = cuda_status(cudaMemset(err, 0, sizeof(unsigned)));
+        if (!s) s = cuda_status(cudaMemsetAsync(err, 0, sizeof(unsigned), stream));
         return s;
     }
     // NQB_E_STALL if a GEMM of the passes so far timed out (synchronises the stream).
@@ -584,7 +589,7 @@ struct Work {
         return st ? st : (h & 2u) ? NQB_E_DEVICE : (h ? NQB_E_STALL : NQB_OK);
     }
     ~Work() {
-        for (void* p : owned) cudaFree(p);
+        for (void* p : owned) dev_free(p, stream);
     }
 };
 
@@ -678,24 +683,24 @@ struct CallScope {  // current device for the call, restored afterwards; one str
     explicit CallScope(int dev) {
         cudaGetDevice(&prev);
         if ((status = cuda_status(cudaSetDevice(dev)))) return;
-        status = cuda_status(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        status = stream_take(&s);
     }
     ~CallScope() {
-        if (s) {
-            cudaStreamSynchronize(s);
-            cudaStreamDestroy(s);
-        }
+        if (s) stream_give(s);
         cudaSetDevice(prev);
     }
 };
 
+// Device buffer of one call, stream-ordered.
 template <class T>
 struct DevBuf {
     T* p = nullptr;
-    int alloc(size_t n) { return cuda_malloc(&p, (n ? n : 1) * sizeof(T)); }
-    ~DevBuf() {
-        if (p) cudaFree(p);
-    }
+    cudaStream_t s;
+    explicit DevBuf(cudaStream_t st) : s(st) {}
+    int alloc(size_t n) { return dev_alloc(&p, (n ? n : 1) * sizeof(T), s); }
+    ~DevBuf() { dev_free(p, s); }
+    DevBuf(const DevBuf&) = delete;
+    DevBuf& operator=(const DevBuf&) = delete;
 };
 
 int refresh_half(nqb_model* m, cudaStream_t s) {
@@ -795,8 +800,8 @@ int nqb_model_predict_ex(const nqb_model* m, const nqb_state* states, uint64_t c
     if (count > 0xFFFFFFFFull) return NQB_E_RANGE;
     CallScope cs(m->device);
     if (cs.status) return cs.status;
-    DevBuf<nqb_state> d_st;
-    DevBuf<float> d_out;
+    DevBuf<nqb_state> d_st(cs.s);
+    DevBuf<float> d_out(cs.s);
     int st = d_st.alloc(count);
     if (!st) st = d_out.alloc(count);
     if (!st) st = cuda_status(cudaMemcpyAsync(d_st.p, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, cs.s));
@@ -812,8 +817,8 @@ int nqb_model_loss_grad(nqb_model* m, const nqb_state* states, const float* targ
     if (count > (1u << 20)) return NQB_E_RANGE;
     CallScope cs(m->device);
     if (cs.status) return cs.status;
-    Work w;
-    DevBuf<nqb_state> d_st;
+    Work w(cs.s);
+    DevBuf<nqb_state> d_st(cs.s);
     int st = w.init((uint32_t)count);
     if (!st) st = d_st.alloc(count);
     if (!st) st = cuda_status(cudaMemcpyAsync(d_st.p, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, cs.s));
@@ -846,11 +851,11 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
     CallScope cs(m->device);
     if (cs.status) return cs.status;
     const uint32_t B = (uint32_t)std::min<uint64_t>(o.batch, count);
-    Work w;
-    DevBuf<nqb_state> d_st;
-    DevBuf<__half> d_X;
-    DevBuf<float> d_t;
-    DevBuf<uint32_t> d_perm;
+    Work w(cs.s);
+    DevBuf<nqb_state> d_st(cs.s);
+    DevBuf<__half> d_X(cs.s);
+    DevBuf<float> d_t(cs.s);
+    DevBuf<uint32_t> d_perm(cs.s);
     int st = w.init(B);
     if (!st) st = d_st.alloc(count);
     if (!st) st = d_X.alloc(count * kIn);

@@ -140,6 +140,12 @@ int launch_plain_refined(const nqb_state* d_states, uint64_t count, unsigned lon
                          cudaStream_t s, unsigned* launches, SchedInfo* info,
                          unsigned long long* d_lane_stats = nullptr);
 
+// A stream of the current device for one call (devmem.cu): an idle one kept from an earlier
+// call, or a new one.  stream_give waits for it and keeps it for later calls; the device it was
+// taken on must be current.
+int stream_take(cudaStream_t* s);
+void stream_give(cudaStream_t s);
+
 // Stream-ordered device allocation from the library's pool on the current device
 // (devmem.cu); release with dev_free on a stream.  Freed memory stays cached for later
 // calls until nqb_trim_device_memory.

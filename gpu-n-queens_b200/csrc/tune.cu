@@ -97,16 +97,13 @@ extern "C" int nqb_tune_count(unsigned n, const unsigned* depths, unsigned n_dep
         unsigned long long* d_out = nullptr;
         ~Held() {
             if (d_out) dev_free(d_out, s);
-            if (s) {
-                cudaStreamSynchronize(s);
-                cudaStreamDestroy(s);
-            }
+            if (s) stream_give(s);
             cudaSetDevice(prev);
         }
     } held;
     cudaGetDevice(&held.prev);
     int st = cuda_status(cudaSetDevice(base.device));
-    if (!st) st = cuda_status(cudaStreamCreateWithFlags(&held.s, cudaStreamNonBlocking));
+    if (!st) st = stream_take(&held.s);
     const cudaStream_t s = held.s;
     if (!st) st = dev_alloc(&held.d_out, 8 * sizeof(unsigned long long) + kBatchedScratchBytes, s);  // results, scratch
     unsigned long long* const d_out = held.d_out;

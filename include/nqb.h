@@ -10,7 +10,7 @@
  * Every entry point returns an NQB_* status code and never exits the process
  * (the reference's FAIL_IF / CHECK_CUDA_ERROR exit; deffinitions.cuh:148-156).
  * Plain pointers and sizes only; no C++ or torch types cross this boundary.
- * Calls are re-entrant: each call owns its own stream and device buffers.
+ * Calls are re-entrant: each call has a stream and device buffers to itself.
  */
 #ifndef NQB_H
 #define NQB_H
@@ -138,7 +138,8 @@ int nqb_device_check(int device);
 
 /* Device buffers of a call (the pool, its level buffers, scratch) come from the library's
  * own stream-ordered memory pool on that device and stay cached for the next call instead
- * of being unmapped; this returns the cached memory of `device` to the driver. */
+ * of being unmapped, and up to 16 idle streams are kept for the next calls; this returns the
+ * cached memory of `device` to the driver and destroys its idle streams. */
 int nqb_trim_device_memory(int device);
 
 /* Test hook for the error paths: makes one allocation of the library fail as if memory had
