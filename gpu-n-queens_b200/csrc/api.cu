@@ -67,6 +67,16 @@ class Scope {
         *p = static_cast<T*>(bufs_.back());
         return NQB_OK;
     }
+    // Takes over a buffer of the stream's: freed with the scope.
+    void hold(void* p) {
+        if (!p) return;
+        try {
+            bufs_.push_back(p);
+        } catch (...) {
+            dev_free(p, stream);
+            throw;
+        }
+    }
     int event(cudaEvent_t* e) {
         events_.push_back(nullptr);
         const int s = cuda_status(cudaEventCreate(&events_.back()));
@@ -94,12 +104,19 @@ nqb_opts resolve(const nqb_opts* o) {
 }
 
 
-// Solves `count` states already on the device (d_states, stack bound `depth`) with the form
-// o.form; fills totals {count, nodes, unit, err} and optional per-state results.  e_start is
-// recorded before any H2D copy so that h2d_ms covers it.
+// A pool that a call builds itself, without reading its sizes back (small_pool_items).
+struct OwnPool {
+    unsigned n, depth;
+    double gen_ms;  // set by the call
+};
+
+// Solves `count` states already on the device (d_states, stack bound `depth`), or those of
+// `pool`, with the form o.form; fills totals {count, nodes, unit, err} and optional per-state
+// results.  e_start is recorded before any H2D copy so that h2d_ms covers it.  NQB_E_RANGE
+// with a pool: it is larger than small_pool took it for.
 int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, unsigned depth, const nqb_opts& o,
                         unsigned long long totals[4], uint64_t* per_state, nqb_stats* st,
-                        uint64_t* per_state_nodes, cudaEvent_t e_start) {
+                        uint64_t* per_state_nodes, cudaEvent_t e_start, OwnPool* pool = nullptr) {
     const bool batched = o.form == NQB_FORM_BATCHED;
     if (o.form != NQB_FORM_PLAIN && !batched) return NQB_E_INVALID;
     if (batched && count > (1ull << 31)) return NQB_E_RANGE;
@@ -121,11 +138,35 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     NQB_TRY(sc.event(&e2));
     NQB_TRY(cuda_status(cudaMemsetAsync(d_out, 0, out_bytes, sc.stream)));
     if (d_per) NQB_TRY(cuda_status(cudaMemsetAsync(d_per, 0, count * sizeof(unsigned long long), sc.stream)));
-    NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
     unsigned launches = 0;
     SchedInfo sched;
+    Refined own;
+    if (pool) {
+        cudaEvent_t e0;
+        NQB_TRY(sc.event(&e0));
+        NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
+        const int s = small_pool_items(pool->n, pool->depth, o.count_unit_nodes && !batched, sc.device, sc.stream,
+                                       d_out, &launches, &own, &count);
+        sc.hold(own.buf);
+        NQB_TRY(s);
+        NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
+        float g = 0.0f;
+        cudaEventSynchronize(e1);
+        cudaEventElapsedTime(&g, e0, e1);
+        pool->gen_ms = g;
+    } else {
+        NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
+    }
     sched.items = count;
-    if (count) {
+    if (pool) {
+        sched.items = own.n;
+        if (batched)
+            NQB_TRY(launch_batched(own.items, own.n, nullptr, nullptr, d_out + 8, kBatchedScratchBytes, d_out, nullptr,
+                                   nullptr, o.block_size, own.stack_depth, sc.device, sc.stream, &launches, d_lanes));
+        else
+            NQB_TRY(launch_plain(own.items, own.n, d_out, nullptr, o.block_size, o.count_unit_nodes != 0,
+                                 own.stack_depth, sc.stream, &launches, d_lanes));
+    } else if (count) {
         if (batched) {
             NQB_TRY(launch_batched_scheduled(d_states, (uint32_t)count, nullptr, d_out + 8, kBatchedScratchBytes, d_out,
                                              d_per, d_per_nodes, o, depth, sc.device, sc.stream, &launches, &sched,
@@ -311,21 +352,29 @@ int nqb_count_ex(unsigned n, unsigned depth, const nqb_opts* opts, uint64_t* cou
         NQB_TRY(solve_host_states(sc, pool, cnt, o, totals, nullptr, stats, nullptr,
                                   n - depth - 1 > 0 ? n - depth - 1 : 1));
     } else {  // build the pool on the GPU: nothing crosses PCIe but the result
-        cudaEvent_t g0, g1;
-        NQB_TRY(sc.event(&g0));
-        NQB_TRY(sc.event(&g1));
-        NQB_TRY(cuda_status(cudaEventRecord(g0, sc.stream)));
-        nqb_state* d_pool = nullptr;
-        uint64_t cnt = 0;
-        NQB_TRY(generate_pool_device(n, depth, sc.stream, &d_pool, &cnt));
-        cudaEventRecord(g1, sc.stream);
-        const int s = solve_device_states(sc, d_pool, cnt, n - depth - 1 > 0 ? n - depth - 1 : 1, o, totals, nullptr,
-                                          stats, nullptr, nullptr);
-        dev_free(d_pool, sc.stream);
+        OwnPool own{n, depth, 0.0};
+        int s = NQB_E_RANGE;
+        if (small_pool(n, depth) && (o.form == NQB_FORM_PLAIN || (!o.model && o.sched_cost == 0))) {
+            s = solve_device_states(sc, nullptr, 0, 0, o, totals, nullptr, stats, nullptr, nullptr, &own);
+            gen_ms = own.gen_ms;
+        }
+        if (s == NQB_E_RANGE) {
+            cudaEvent_t g0, g1;
+            NQB_TRY(sc.event(&g0));
+            NQB_TRY(sc.event(&g1));
+            NQB_TRY(cuda_status(cudaEventRecord(g0, sc.stream)));
+            nqb_state* d_pool = nullptr;
+            uint64_t cnt = 0;
+            NQB_TRY(generate_pool_device(n, depth, sc.stream, &d_pool, &cnt));
+            cudaEventRecord(g1, sc.stream);
+            s = solve_device_states(sc, d_pool, cnt, n - depth - 1 > 0 ? n - depth - 1 : 1, o, totals, nullptr, stats,
+                                    nullptr, nullptr);
+            dev_free(d_pool, sc.stream);
+            float g = 0.0f;
+            if (s == NQB_OK) cudaEventElapsedTime(&g, g0, g1);
+            gen_ms = g;
+        }
         NQB_TRY(s);
-        float g = 0.0f;
-        cudaEventElapsedTime(&g, g0, g1);
-        gen_ms = g;
     }
     *count = totals[0];
     if (stats) {

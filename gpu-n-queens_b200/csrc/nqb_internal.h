@@ -100,6 +100,14 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
                  unsigned stack_depth, int device, cudaStream_t s, unsigned long long* d_totals,
                  unsigned long long* d_board_nodes, unsigned* launches, Refined* out);
 
+// The (n, depth) pool of a count, split further when it is small, without reading any level's
+// size back: for pools of which small_pool(n, depth) says that they fit refine_items' buffers.
+// *states is the pool's size, `out` the items to search (in no particular order).  Counts like
+// refine_items.  NQB_E_RANGE: the pool did not fit after all.
+bool small_pool(unsigned n, unsigned depth);
+int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
+                     unsigned* launches, Refined* out, uint64_t* states);
+
 // Items after learned scheduling: the caller's arrays, or split / ordered device copies
 // owned by the schedule until release() (stream-ordered frees).
 struct Schedule {

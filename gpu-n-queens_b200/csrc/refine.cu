@@ -1,4 +1,4 @@
-// Splits the items of a launch that has too few of them.
+// Splits the items of a launch that has too few of them, and builds the pools of small counts.
 //
 // A search kernel keeps its lanes busy only while it has several items a lane: with fewer,
 // the time goes into handing pieces of long subtrees from lane to lane and from warp to warp.
@@ -23,6 +23,7 @@
 // at one item a lane leaves N=19 at depth 4 at 165 ms and the uneven boards at 239 ms, against
 // 147.5 and 209 ms (same box) at two; at four, calls move within 4% either way.
 #include <algorithm>
+#include <cmath>
 
 #include "nqb_internal.h"
 #include "search_step.cuh"
@@ -37,6 +38,8 @@ constexpr uint32_t kMinSplitFree = 8;      // items with fewer free columns are 
 constexpr uint32_t kSplitSpread = 3;
 constexpr unsigned kMaxLevels = 4;
 constexpr unsigned kThreads = 256;
+constexpr unsigned kMaxRecords = NQB_MAX_N + kMaxLevels;  // a pool's levels, then the split's
+constexpr size_t kHeadBytes = 2048;
 
 struct Level {
     const uint4* items;
@@ -76,9 +79,11 @@ __global__ void first_kernel(const uint4* __restrict__ items, const uint32_t* __
     }
 }
 
-// One level: in -> out, or `in` handed on.  UNIT: children whose row has exactly one candidate
+// One level: in -> out, or `in` handed on.  COUNT: the candidates of split items are counted as
+// nodes (a level below the pool; the levels that build the pool split everything and count
+// nothing).  UNIT: children whose row has exactly one candidate
 // are counted as unit placements (a search kernel takes an item's first row for a start row).
-template <bool UNIT>
+template <bool COUNT, bool UNIT>
 __global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict__ in, Level* __restrict__ out,
                                                          uint4* __restrict__ to, uint32_t* __restrict__ to_board,
                                                          uint32_t cut, uint32_t next_cut, uint32_t enough,
@@ -86,12 +91,12 @@ __global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict
                                                          unsigned long long* __restrict__ board_nodes) {
     const uint32_t n = in->n;
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
-    if (n >= enough || in->next > kCapItems || in->next == n) {
+    if (in->next > kCapItems || (COUNT && (n >= enough || in->next == n))) {
         if (first) {
             out->items = in->items;
             out->board = in->board;
             out->n = n;
-            out->next = n;  // the levels after this one hand it on too
+            out->next = COUNT ? n : ~0ull;  // the levels after this one hand it on too
             out->done = in->done;
         }
         return;
@@ -109,7 +114,7 @@ __global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict
         const uint32_t nc = free_columns(s);
         const bool split = valid && (uint32_t)__popc(nc) >= cut;
         const uint32_t kids = split ? living(s, nc) : 0u;
-        if (split) {
+        if (COUNT && split) {
             const uint32_t placed = __popc(nc & ~(s.y | s.z));
             nodes += placed;
             if (board_nodes && placed) atomicAdd(board_nodes + id, (unsigned long long)placed);
@@ -157,6 +162,60 @@ __global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict
     }
 }
 
+// The first level of a pool: the row-0 placements of the left half whose next row has a
+// candidate, weight 2 left of centre and 1 for the middle column of an odd board
+// (GPU_NQueens.cu:354-357).  Also clears the level records.
+__global__ void seed_kernel(uint32_t n, uint32_t next_cut, uint4* __restrict__ items, Level* __restrict__ lv) {
+    const uint32_t lane = threadIdx.x;  // one warp; n <= 31
+    for (uint32_t w = lane; w < kMaxRecords * sizeof(Level) / 4; w += 32) reinterpret_cast<uint32_t*>(lv)[w] = 0;
+    __syncwarp();
+    const uint32_t b = 1u << lane;
+    const uint4 s = make_uint4(b, b << 1, b >> 1, 1u | (n << 8) | ((lane < (n >> 1) ? 2u : 1u) << 16));
+    const bool kept = lane < (n + 1) / 2 && (free_columns(s) & ~(s.y | s.z));
+    const uint32_t all = __ballot_sync(kFull, kept);
+    if (kept) items[__popc(all & (b - 1u))] = s;
+    const uint32_t made = (uint32_t)warp_sum_u64(kept ? made_of(s, next_cut) : 0);
+    if (lane == 0) {
+        lv->items = items;
+        lv->n = __popc(all);
+        lv->next = made;
+    }
+}
+
+// Free columns from which level `level` of a split splits, of items that have max_free at most.
+uint32_t cut_of(uint32_t max_free, unsigned level) {
+    const uint32_t top = max_free - level;
+    return std::max(kMinSplitFree, top > kSplitSpread ? top - kSplitSpread : 0u);
+}
+
+unsigned split_levels(uint32_t max_free) {
+    return max_free <= kMinSplitFree ? 0 : std::min(kMaxLevels, max_free - kMinSplitFree);
+}
+
+// The buffers of a call's levels: the records, then two item buffers used in turn.
+struct Levels {
+    Level* records;
+    uint4* items[2];
+    uint32_t* board[2];
+    int take(bool boards, cudaStream_t s, Refined* out) {
+        static_assert(kMaxRecords * sizeof(Level) <= kHeadBytes, "the level records' room");
+        const size_t item_bytes = (size_t)kCapItems * sizeof(uint4);
+        const size_t board_bytes = boards ? (size_t)kCapItems * sizeof(uint32_t) : 0;
+        NQB_TRY(dev_alloc_bytes(&out->buf, kHeadBytes + 2 * (item_bytes + board_bytes), s));
+        out->stream = s;
+        char* at = static_cast<char*>(out->buf);
+        records = reinterpret_cast<Level*>(at);
+        at += kHeadBytes;
+        for (int k = 0; k < 2; ++k) {
+            items[k] = reinterpret_cast<uint4*>(at);
+            at += item_bytes;
+            board[k] = boards ? reinterpret_cast<uint32_t*>(at) : nullptr;
+            at += board_bytes;
+        }
+        return NQB_OK;
+    }
+};
+
 }  // namespace
 
 void Refined::release() {
@@ -175,33 +234,19 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
     NQB_TRY(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)));
     const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;  // 36 warps of an SM's stack memory
     const uint32_t max_free = stack_depth + 1;
-    if (n >= enough || max_free <= kMinSplitFree) return NQB_OK;
-    const unsigned levels = std::min(kMaxLevels, max_free - kMinSplitFree);
-    auto cut_of = [&](unsigned level) {  // free columns from which a level splits
-        const uint32_t top = max_free - level;
-        return std::max(kMinSplitFree, top > kSplitSpread ? top - kSplitSpread : 0u);
-    };
-    boards = boards || d_board;
-    const size_t item_bytes = (size_t)kCapItems * sizeof(uint4);
-    const size_t board_bytes = boards ? (size_t)kCapItems * sizeof(uint32_t) : 0;
-    const size_t head = (kMaxLevels + 1) * sizeof(Level) + 64;
-    void* mem = nullptr;
-    NQB_TRY(dev_alloc_bytes(&mem, 512 + 2 * (item_bytes + board_bytes), s));
-    static_assert((kMaxLevels + 1) * sizeof(Level) + 64 <= 512, "the level records have 512 bytes");
-    out->buf = mem;
-    out->stream = s;
-    char* const base = static_cast<char*>(mem);
-    Level* const lv = reinterpret_cast<Level*>(base);
-    NQB_TRY(cuda_status(cudaMemsetAsync(lv, 0, head, s)));
+    const unsigned levels = split_levels(max_free);
+    if (n >= enough || levels == 0) return NQB_OK;
+    Levels b;
+    NQB_TRY(b.take(boards || d_board, s, out));
+    Level* const lv = b.records;
+    NQB_TRY(cuda_status(cudaMemsetAsync(lv, 0, (levels + 1) * sizeof(Level), s)));
     const unsigned grid0 = std::max(1u, std::min((n + kThreads - 1) / kThreads, 4u * (unsigned)sms));
-    first_kernel<<<grid0, kThreads, 0, s>>>(reinterpret_cast<const uint4*>(d_items), d_board, n, cut_of(0), lv);
+    first_kernel<<<grid0, kThreads, 0, s>>>(reinterpret_cast<const uint4*>(d_items), d_board, n, cut_of(max_free, 0),
+                                            lv);
     for (unsigned k = 0; k < levels; ++k) {
-        char* const to = base + 512 + (k & 1) * (item_bytes + board_bytes);
-        uint4* const to_items = reinterpret_cast<uint4*>(to);
-        uint32_t* const to_board = boards ? reinterpret_cast<uint32_t*>(to + item_bytes) : nullptr;
-        auto kern = unit ? level_kernel<true> : level_kernel<false>;
-        kern<<<4 * sms, kThreads, 0, s>>>(lv + k, lv + k + 1, to_items, to_board, cut_of(k), cut_of(k + 1), enough,
-                                          d_totals, d_board_nodes);
+        auto kern = unit ? level_kernel<true, true> : level_kernel<true, false>;
+        kern<<<4 * sms, kThreads, 0, s>>>(lv + k, lv + k + 1, b.items[k & 1], b.board[k & 1], cut_of(max_free, k),
+                                          cut_of(max_free, k + 1), enough, d_totals, d_board_nodes);
     }
     NQB_TRY(cuda_status(cudaGetLastError()));
     if (launches) *launches += 1 + levels;
@@ -212,8 +257,59 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
     out->board = last.board;
     out->n = last.n;
     // Every item with more than max_free - done free columns has been split (a level's cut is
-    // at most its largest), unless the cut was held at kMinSplitFree.
+    // at most its largest).
     out->stack_depth = std::max(stack_depth > last.done ? stack_depth - last.done : 1u, 1u);
+    return NQB_OK;
+}
+
+namespace {
+// Estimated children per state of a level with `row` queens placed: 0.8 to 1.9 times the real
+// ones over all levels to a depth of n / 2, n = 8..21.
+double children_estimate(unsigned n, unsigned row) { return n * std::pow(1.0 - (double)row / n, 2.4); }
+}  // namespace
+
+bool small_pool(unsigned n, unsigned depth) {
+    double size = (n + 1) / 2;
+    for (unsigned r = 1; r < depth; ++r)
+        if ((size *= children_estimate(n, r)) > 0.8 * kCapItems) return false;
+    return true;
+}
+
+int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
+                     unsigned* launches, Refined* out, uint64_t* states) {
+    *states = 0;
+    int sms = 0;
+    NQB_TRY(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)));
+    const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;
+    const uint32_t max_free = n - depth;
+    const unsigned levels = split_levels(max_free), all = depth - 1 + levels;
+    Levels b;
+    NQB_TRY(b.take(false, s, out));
+    Level* const lv = b.records;
+    auto cut = [&](unsigned k) { return k < depth - 1 ? 0u : cut_of(max_free, k - (depth - 1)); };
+    seed_kernel<<<1, 32, 0, s>>>(n, all ? cut(0) : 0u, b.items[1], lv);
+    double size = (n + 1) / 2;  // of the level's input, for the grid
+    for (unsigned k = 0; k < all; ++k) {
+        auto kern = k < depth - 1 ? level_kernel<false, false>
+                                  : unit ? level_kernel<true, true> : level_kernel<true, false>;
+        const unsigned grid = (unsigned)std::min(4.0 * sms, size / kThreads + 1.0);
+        kern<<<grid, kThreads, 0, s>>>(lv + k, lv + k + 1, b.items[k & 1], nullptr, cut(k), cut(k + 1), enough,
+                                       d_totals, nullptr);
+        size *= children_estimate(n, k + 1);
+    }
+    NQB_TRY(cuda_status(cudaGetLastError()));
+    if (launches) *launches += 1 + all;
+    Level rec[kMaxRecords];
+    NQB_TRY(cuda_status(cudaMemcpyAsync(rec, lv, (all + 1) * sizeof(Level), cudaMemcpyDeviceToHost, s)));
+    NQB_TRY(cuda_status(cudaStreamSynchronize(s)));
+    if (rec[depth - 1].done != depth - 1) return NQB_E_RANGE;  // a level of the pool did not fit
+    const Level& last = rec[all];
+    const unsigned split = last.done - (depth - 1);
+    *states = rec[depth - 1].n;
+    out->items = reinterpret_cast<const nqb_state*>(last.items);
+    out->board = nullptr;
+    out->n = last.n;
+    out->stack_depth = max_free > split + 1 ? max_free - split - 1 : 1;
     return NQB_OK;
 }
 

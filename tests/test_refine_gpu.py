@@ -44,3 +44,23 @@ def test_shallow_pools_keep_counts_nodes_and_unit_nodes(nqb, nqo, n, d):
     assert c == b and st["nodes"] == sb["nodes"] and st["states"] == sb["states"]
     if want:
         assert (c, st["nodes"], st["unit_nodes"]) == (want["count"], want["nodes"], want["unit"])
+
+
+@pytest.mark.parametrize("n", [4, 5, 6, 7, 8, 11])
+def test_every_pool_depth_of_small_boards(nqb, nqo, n):
+    # the pool built without read-backs: each depth's size, and the count below it
+    for d in range(1, n):
+        for form in (nqb.FORM_PLAIN, nqb.FORM_BATCHED):
+            c, st = nqb.count_ex(n, d, form=form)
+            assert st["states"] == nqb.pool_size(n, d), (n, d, form)
+            want = nqb.generate_pool(n, d)
+            total, nodes = nqo.solve_states(want) if len(want) else (np.zeros(1, dtype=np.uint64), 0)
+            assert c == int(np.sum(total)) and st["nodes"] == nodes, (n, d, form)
+
+
+def test_pools_around_the_buffers_size(nqb):
+    # the largest pools built without read-backs and the smallest built with them
+    for n, d in [(17, 6), (17, 7), (18, 6), (15, 7), (15, 9), (16, 7), (16, 8), (16, 15)]:
+        c, st = nqb.count_ex(n, d, form=nqb.FORM_BATCHED)
+        assert st["states"] == nqb.pool_size(n, d)
+        assert c == {15: 2279184, 16: 14772512, 17: 95815104, 18: 666090624}[n]
