@@ -62,12 +62,15 @@ constexpr int kUnroll = NQB_BATCHED_UNROLL;
 constexpr int kRefresh = 24;  // steps between refreshes of the lanes' sentinels
 static_assert(kRefresh <= kMaxParkedSteps, "a parked lane would pop past its sentinel");
 constexpr uint32_t kEpoch = (1u << 27) / kUnroll;  // rounds between folds: 31 nodes x kUnroll x kEpoch < 2^32
-constexpr uint32_t kDonateEvery = 16;        // rounds between a busy warp's looks at the hungry count
-// The spread instance (launches with fewer items than lanes) looks 8x less often.  Measured on
-// coarse pools against every 16 and 64 rounds: N=19 d=4 215 / 205 / 196 ms, N=20 d=4 1400 /
-// 1385 / 1373 ms, the 65,536 uneven boards 1836 ms at 64 and 1824 ms at 128; only the smallest
-// launch (N=17 d=3, 9 ms) is faster at 64, by 0.5 ms.  256 is no better than 128.
-constexpr uint32_t kDonateEverySpread = 8 * kDonateEvery;
+// Rounds between a busy warp's looks at the hungry count.  A look that finds hungry warps gives
+// pieces away that are often small, so looking often costs more than the waits it saves: with
+// few items a lane every 128 rounds is best (1/16 of the N=20 depth-6 pool, one item a lane:
+// 16 / 32 / 64 / 128 / 512 rounds 91.3 / 88.4 / 86.0 / 84.4 / 85.9 ms; the N=18 depth-5 pool
+// 28.2 / 26.7 / 26.3 / 26.4 / 29.0 ms), and from kPlentyItems a lane on the queue itself keeps
+// the warps busy to the end (N=18 at depth 6 16 / 64 / 128 / 512 rounds 18.45 / 18.59 / 18.65 /
+// 18.40 ms).
+constexpr uint32_t kDonateEvery = 128, kDonateEveryPlenty = 512;
+constexpr uint64_t kPlentyItems = 4;
 
 // Error flags written to out[3].
 constexpr unsigned long long kErrStack = 1ull;  // an item needed a deeper stack than provided
@@ -85,6 +88,7 @@ struct BatchArgs {
     uint4* ring;                          // steal ring (2 x uint4 per slot), turn words zero at launch
     uint32_t ring_cap;                    // slots, a power of two; 0 = no stealing across warps
     uint32_t ring_shift;                  // log2(ring_cap)
+    uint32_t donate_every;                // rounds between looks at the hungry count
     uint32_t wait_limit;                  // polls without progress before a wait gives up
     unsigned long long* out;              // {weighted count, nodes, 0, error flags}
     unsigned long long* per_board;        // optional: weighted count per board
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
         // seen the item queue run dry itself (hungry warps exist only once it has).  The tail
         // only moves by a compare-and-swap against the snapshot the room was computed from,
         // so the ring never holds more than half its slots and a producer never waits a lap.
-        if (a.ring_cap && ++rounds == (SPREAD ? kDonateEverySpread : kDonateEvery)) {
+        if (a.ring_cap && ++rounds == a.donate_every) {
             rounds = 0;
             const uint32_t donors = __ballot_sync(kFull, s.sp != base);
             if (donors) {
@@ -369,7 +373,7 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
 }
 
 template <int BLOCK, bool LANES>
-int launch_batched_t(const BatchArgs& a, int device, cudaStream_t stream, unsigned* launches) {
+int launch_batched_t(BatchArgs a, int device, cudaStream_t stream, unsigned* launches) {
     const size_t smem = (size_t)(a.stack_depth + 1) * BLOCK * sizeof(uint4);
     if (smem > 227 * 1024) return NQB_E_RANGE;
     auto kern = batched_search_kernel<BLOCK, LANES, false>;
@@ -388,7 +392,9 @@ int launch_batched_t(const BatchArgs& a, int device, cudaStream_t stream, unsign
     // One wave of blocks; with stealing, fewer items than lanes still fill the whole GPU.
     const uint64_t wave = (uint64_t)sms * per_sm;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, a.ring_cap ? wave : std::min<uint64_t>(wave, need));
-    if (a.ring_cap && (uint64_t)a.n_items < (uint64_t)grid * BLOCK)
+    const uint64_t lanes = (uint64_t)grid * BLOCK;
+    a.donate_every = a.n_items >= kPlentyItems * lanes ? kDonateEveryPlenty : kDonateEvery;
+    if (a.ring_cap && a.n_items < lanes)
         spread<<<grid, BLOCK, smem, stream>>>(a);
     else
         kern<<<grid, BLOCK, smem, stream>>>(a);
