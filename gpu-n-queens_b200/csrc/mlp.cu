@@ -12,7 +12,8 @@
 //   dy = 2 (y - t)      dZ2 = dy w3^T * gelu'(Z2 + b2)      dH1 = dZ2 W2^T
 //   dZ1 = dH1 * gelu'(Z1 + b1)
 //   dW2 = H1^T dZ2 / B  dW1 = X^T dZ1 / B  dw3 = H2^T dy / B  (bias grads: column sums / B)
-// All GEMMs go through one tcgen05 kernel with arbitrary operand strides (gemm_tc).
+// One kernel runs the whole step for 128 rows at a time, with every intermediate in shared or
+// tensor memory (train_kernel); a second one adds up the blocks' gradients and applies Adam.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -58,11 +59,22 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
 // Byte offset of K step k (16 elements) inside an operand tile.
 __device__ __forceinline__ uint32_t kstep_offset(int k) { return (uint32_t)(k >> 2) * kAtomBytes + (uint32_t)(k & 3) * 32u; }
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumulate) {
+// The same tile read the other way round (MN-major): its rows are the K index and its columns,
+// contiguous in memory, the M or N index.  64 columns are one 128-byte row of an atom; the
+// next 64 are kAtomBytes on (leading offset), the next 8 rows 1024 bytes (stride offset).  A K
+// step of 16 rows is 2048 bytes.
+__device__ __forceinline__ uint64_t sw128_desc_mn(uint32_t addr) {
+    return sw128_desc(addr) - ((uint64_t)1u << 16) + ((uint64_t)(kAtomBytes >> 4) << 16);
+}
+constexpr uint32_t kKstepRows = 16u * 128u;
+constexpr uint32_t kMnA = 1u << 15, kMnB = 1u << 16;  // instruction descriptor: A, B MN-major
+
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumulate,
+                                         uint32_t idesc = kIdesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %4, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(accumulate), "r"(kIdesc), "r"(0u));
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(accumulate), "r"(idesc), "r"(0u));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -118,274 +130,11 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// ---- GEMM: C (M x N, fp32, row-major ldc) = alpha * A x B, on tcgen05 ----------------------
-// A(i, k) = A[i * sai + k * sak], B(k, j) = B[k * sbk + j * sbj], fp16; N <= 128.  A block
-// owns 128 rows of C and a range of K; every 64-element K step is loaded into swizzled
-// shared memory (a 16-byte vector per chunk when K is contiguous and aligned, else 8
-// element loads that are coalesced across the block's rows) and multiplied as four K=16
-// MMAs into a 128 x 128 fp32 tensor-memory accumulator.  With several K ranges (the weight
-// gradients, K = batch rows) each block adds its partial product with fp32 atomics into a
-// zeroed C.  The shared-memory request caps residency at 3 blocks (384 tensor-memory
-// columns) per SM.
-constexpr uint32_t kGemmSmem = 72 * 1024;
-constexpr int kGemmK = 64;
-
-__device__ __forceinline__ void load_chunk(const __half* __restrict__ p, long stride_k, int valid, bool vec,
-                                           uint32_t q[4]) {
-    if (vec && valid == 8) {
-        const uint4 v = *reinterpret_cast<const uint4*>(p);
-        q[0] = v.x, q[1] = v.y, q[2] = v.z, q[3] = v.w;
-        return;
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const __half a = 2 * e < valid ? p[(long)(2 * e) * stride_k] : __float2half(0.0f);
-        const __half b = 2 * e + 1 < valid ? p[(long)(2 * e + 1) * stride_k] : __float2half(0.0f);
-        __half2 h = __halves2half2(a, b);
-        q[e] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
-
-__global__ void __launch_bounds__(128) gemm_tc(const __half* __restrict__ A, long sai, long sak, bool a_vec,
-                                               const __half* __restrict__ B, long sbk, long sbj, bool b_vec,
-                                               float* __restrict__ C, long ldc, int M, int N, int K, int k_per_block,
-                                               float alpha, bool atomic, unsigned* __restrict__ err) {
-    extern __shared__ unsigned char smem_raw[];
-    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
-    const uint32_t base = (raw + 1023u) & ~1023u;
-    const uint32_t as = base, bs = base + kAtomBytes, bar = base + 2 * kAtomBytes, tmem_slot = bar + 8;
-    const uint32_t t = threadIdx.x, warp = t >> 5;
-    const int m0 = blockIdx.x * kTileRows;
-    const int kb = blockIdx.y * k_per_block, ke = min(K, kb + k_per_block);
-    if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    uint32_t tmem = 0;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
-    uint32_t phase = 0;
-    bool failed = false, undrained = false;
-    const int i = m0 + (int)t;  // this thread's row of A and of C
-    const int j = (int)t;       // this thread's row of B (column of C)
-    for (int k0 = kb; k0 < ke && !failed; k0 += kGemmK) {
-#pragma unroll
-        for (uint32_t c = 0; c < kGemmK / 8; ++c) {
-            const int k = k0 + (int)c * 8;
-            const int valid = max(0, min(8, ke - k));
-            uint32_t q[4] = {0u, 0u, 0u, 0u};
-            if (i < M) load_chunk(A + (long)i * sai + (long)k * sak, sak, valid, a_vec, q);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(as + sw128_chunk(t, c)), "r"(q[0]),
-                         "r"(q[1]), "r"(q[2]), "r"(q[3])
-                         : "memory");
-            q[0] = q[1] = q[2] = q[3] = 0u;
-            if (j < N) load_chunk(B + (long)k * sbk + (long)j * sbj, sbk, valid, b_vec, q);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(bs + sw128_chunk(t, c)), "r"(q[0]),
-                         "r"(q[1]), "r"(q[2]), "r"(q[3])
-                         : "memory");
-        }
-        proxy_fence();
-        tc_fence_before();
-        __syncthreads();
-        if (t == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-                umma_f16(tmem, sw128_desc(as + ks * 32u), sw128_desc(bs + ks * 32u), (k0 > kb || ks > 0) ? 1u : 0u);
-            umma_commit(bar);
-        }
-        const bool ok = mbar_wait(bar, phase);
-        if (__syncthreads_or(!ok)) {  // timed out: drain the MMAs in flight (bounded), then leave
-            undrained = !__syncthreads_and(mbar_wait(bar, phase));
-            failed = true;
-            break;
-        }
-        phase ^= 1u;  // the shared tiles are free again once the MMAs are done
-    }
-    if (!failed && kb < ke) {
-        // Epilogue: 32 accumulator columns at a time go through shared memory (the operand
-        // tiles are free now), [128 rows][33 floats], so that a warp then writes 32
-        // consecutive floats of one row of C per store.
-        tc_fence_after();
-        const uint32_t my_lanes = tmem + ((warp * 32u) << 16);
-        float* stage = reinterpret_cast<float*>(smem_raw + (base - raw));
-        constexpr int kLd = 33;  // padded row: column reads of the staging tile avoid bank conflicts
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-            float v[32];
-            tmem_ld16(my_lanes + (uint32_t)c0, v);
-            tmem_ld16(my_lanes + (uint32_t)c0 + 16u, v + 16);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) stage[t * kLd + e] = v[e];
-            __syncthreads();
-            const int lane = (int)(t & 31u), col = c0 + lane;
-            for (int r = (int)warp; r < kTileRows; r += 4) {
-                const int row = m0 + r;
-                if (row < M && col < N) {
-                    float* p = C + (long)row * ldc + col;
-                    const float x = alpha * stage[r * kLd + lane];
-                    if (atomic) atomicAdd(p, x);
-                    else *p = x;
-                }
-            }
-            __syncthreads();
-        }
-    }
-    // bit 0: a completion wait timed out; bit 1: the drain timed out too, so products may still
-    // have been in flight when the tensor memory was freed
-    if (failed && t == 0) atomicOr(err, undrained ? 3u : 1u);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-}
-
-// C = alpha * A x B (the only form training uses; beta must be 0).  `err`: device word the
-// kernel sets when an MMA completion wait times out.
-int gemm(const __half* A, long sai, long sak, const __half* B, long sbk, long sbj, float* C, long ldc, int M, int N,
-         int K, float alpha, float beta, unsigned* err, cudaStream_t s) {
-    if (M <= 0 || N <= 0 || K <= 0) return NQB_OK;
-    if (beta != 0.0f || N > 128) return NQB_E_INVALID;
-    NQB_TRY(cuda_status(cudaFuncSetAttribute(gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem)));
-    auto vec_ok = [](const __half* p, long s_row, long s_k) {
-        return s_k == 1 && ((uintptr_t)p & 15u) == 0 && (s_row * (long)sizeof(__half)) % 16 == 0;
-    };
-    const bool a_vec = vec_ok(A, sai, sak), b_vec = vec_ok(B, sbj, sbk);
-    const int m_tiles = (M + kTileRows - 1) / kTileRows;
-    // split K when it is long (the weight gradients): at least 256 K per block
-    int splits = 1;
-    if (K > 256) splits = std::min((K + 255) / 256, std::max(1, 148 * 3 / m_tiles));
-    const int per = ((K + splits - 1) / splits + kGemmK - 1) / kGemmK * kGemmK;
-    splits = (K + per - 1) / per;
-    if (splits > 1)  // partial products are added into a zeroed C
-        NQB_TRY(cuda_status(
-            cudaMemset2DAsync(C, (size_t)ldc * sizeof(float), 0, (size_t)N * sizeof(float), (size_t)M, s)));
-    const dim3 grid(m_tiles, splits);
-    gemm_tc<<<grid, kTileRows, kGemmSmem, s>>>(A, sai, sak, a_vec, B, sbk, sbj, b_vec, C, ldc, M, N, K, per, alpha,
-                                              splits > 1, err);
-    return cuda_status(cudaGetLastError());
-}
-
-// ---- elementwise and reduction kernels -------------------------------------------------
-__global__ void features_kernel(const uint4* __restrict__ st, const uint32_t* __restrict__ rows, uint32_t n_rows,
-                                __half* __restrict__ X) {
+// ---- features and fp16 weights ------------------------------------------------------------
+__global__ void features_kernel(const uint4* __restrict__ st, uint64_t n_rows, __half* __restrict__ X) {
     const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)n_rows * kIn) return;
-    const uint32_t i = (uint32_t)(e / kIn), j = (uint32_t)(e % kIn);
-    const uint4 s = st[rows ? rows[i] : i];
-    X[e] = __float2half(feature(s, (int)j));
-}
-
-// H = gelu(Z + b) (fp16), Zb = Z + b kept for the backward pass.
-__global__ void bias_gelu_kernel(const float* __restrict__ Z, const float* __restrict__ b, uint32_t rows,
-                                 float* __restrict__ Zb, __half* __restrict__ H) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)rows * kH) return;
-    const float z = Z[e] + b[e % kH];
-    Zb[e] = z;
-    H[e] = __float2half(gelu(z));
-}
-
-// y_i = H2_i . w3 + b3 (one warp per row).
-__global__ void head_kernel(const __half* __restrict__ H2, const float* __restrict__ w3, const float* __restrict__ b3,
-                            uint32_t rows, float* __restrict__ y) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    float s = 0.0f;
-    for (int j = lane; j < kH; j += 32) s += __half2float(H2[(uint64_t)row * kH + j]) * w3[j];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) y[row] = s + b3[0];
-}
-
-// dy = 2 (y - t); the squared error is summed into loss[0].
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ t, uint32_t rows,
-                            float* __restrict__ dy, float* __restrict__ loss) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float e2 = 0.0f;
-    if (i < rows) {
-        const float d = y[i] - t[i];
-        dy[i] = 2.0f * d;
-        e2 = d * d;
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) e2 += __shfl_xor_sync(0xFFFFFFFFu, e2, o);
-    if ((threadIdx.x & 31) == 0 && e2 != 0.0f) atomicAdd(loss, e2);
-}
-
-// dZ2 = dy_i * w3_j * gelu'(Zb2_ij), fp16.
-__global__ void dz2_kernel(const float* __restrict__ dy, const float* __restrict__ w3, const float* __restrict__ Zb2,
-                           uint32_t rows, __half* __restrict__ dZ2) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)rows * kH) return;
-    dZ2[e] = __float2half(dy[e / kH] * w3[e % kH] * gelu_grad(Zb2[e]));
-}
-
-// dZ1 = dH1 * gelu'(Zb1), fp16.
-__global__ void dz1_kernel(const float* __restrict__ dH1, const float* __restrict__ Zb1, uint32_t rows,
-                           __half* __restrict__ dZ1) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)rows * kH) return;
-    dZ1[e] = __float2half(dH1[e] * gelu_grad(Zb1[e]));
-}
-
-// out[j] = scale * sum_i D[i][j] (D fp16 rows x 128); with dy != null: scale * sum_i dy_i D[i][j].
-__global__ void colsum_kernel(const __half* __restrict__ D, const float* __restrict__ dy, uint32_t rows, float scale,
-                              float* __restrict__ out) {
-    const int j = threadIdx.x;  // blockDim = 128
-    float s = 0.0f;
-    for (uint32_t i = blockIdx.x; i < rows; i += gridDim.x) {
-        const float v = __half2float(D[(uint64_t)i * kH + j]);
-        s += dy ? v * dy[i] : v;
-    }
-    atomicAdd(out + j, s * scale);
-}
-
-__global__ void sum_kernel(const float* __restrict__ v, uint32_t n, float scale, float* __restrict__ out) {
-    float s = 0.0f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += v[i];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, s * scale);
-}
-
-__global__ void gather_f16_rows(const __half* __restrict__ X, const uint32_t* __restrict__ rows, uint32_t n_rows,
-                                __half* __restrict__ out) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)n_rows * kIn) return;
-    out[e] = X[(uint64_t)rows[e / kIn] * kIn + e % kIn];
-}
-
-__global__ void gather_f32(const float* __restrict__ v, const uint32_t* __restrict__ rows, uint32_t n,
-                           float* __restrict__ out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = v[rows[i]];
-}
-
-// Adam (Kingma & Ba 2015) on the flat fp32 parameters; refreshes the fp16 copies of W1, W2.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ grad, float* __restrict__ m,
-                            float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1, float c2,
-                            __half* __restrict__ w1h, __half* __restrict__ w2h) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = grad[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float w = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    p[i] = w;
-    if (i < kW1Size) w1h[i] = __float2half(w);
-    else if (i >= kW2 && i < kB2) w2h[i - kW2] = __float2half(w);
+    if (e >= n_rows * kIn) return;
+    X[e] = __float2half(feature(st[e / kIn], (int)(e % kIn)));
 }
 
 __global__ void to_half_kernel(const float* __restrict__ p, __half* __restrict__ w1h, __half* __restrict__ w2h) {
@@ -536,13 +285,342 @@ __global__ void __launch_bounds__(128) predict_kernel(const uint4* __restrict__ 
     }
 }
 
-// Device buffers of one training or gradient pass over batches of up to `cap` rows.
+// ---- one training step (tcgen05) ------------------------------------------------------------
+// A block of 16 warps takes 128 rows of the batch through the whole step.  Thread (quad, lane,
+// group): row 32 quad + lane of the tile (tensor-memory lane 32 quad + lane, which a warp may
+// read only in its quad), hidden columns 32 group .. 32 group + 31.  Both weight matrices and
+// the row tiles X, H1, dZ2 and H2 (then dZ1) lie in shared memory as 128 x 128 fp16 tiles,
+// rows contiguous; a product reads a tile along its rows or its columns as it needs (K-major
+// or MN-major), so nothing is transposed.  The accumulators have 128 tensor-memory columns
+// each: Z1; Z2, then dH1; dW2 and dW1, which go on over the block's tiles.  gelu' of both
+// layers stays in registers between the passes, so each activation's tanh is computed once.
+// A block writes its share of every gradient to a slot of its own (GradParts) and the
+// optimizer kernel adds the slots up in a fixed order: no atomics, and two runs on the same
+// inputs give the same weights.
+//
+// What bounds it: the tanh of 256 activations a row and the waits of one tile's chain of
+// products (32 blocks at the default batch of 4096).  As 5 GEMMs, 10 elementwise or reducing
+// kernels and 2 gathers through global memory the step took 230 us on the device (two thirds of
+// it in the GEMMs, 20-50 us each); two epochs over 65,536 samples, whole call: 6.75 ms before,
+// 1.51 ms now.
+constexpr uint32_t kTrainThreads = 512;
+constexpr uint32_t kTrainTmem = 512;
+constexpr uint32_t kTrainFloats = 3 * kH + 4 + 4 * kTileRows + kTileRows;  // b1 b2 w3 b3 | y partials | dy
+constexpr size_t kTrainSmem = 1024 /* alignment slack */ + 6 * kOpBytes + kTrainFloats * sizeof(float) + 16;
+
+// Gradients of the blocks, one slot a block; tail: {gradient of b3, squared error}.
+struct GradParts {
+    float *w1, *b1, *w2, *b2, *w3, *tail;
+};
+
+__device__ __forceinline__ float half_at(uint32_t tile, uint32_t r, uint32_t c) {
+    unsigned short h;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(tile + sw128_chunk(r, c >> 3) + (c & 7u) * 2u));
+    return __half2float(__ushort_as_half(h));
+}
+
+__device__ __forceinline__ void store_chunk(uint32_t tile, uint32_t r, uint32_t j, uint4 q) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + sw128_chunk(r, j)), "r"(q.x), "r"(q.y),
+                 "r"(q.z), "r"(q.w)
+                 : "memory");
+}
+
+// gelu and its derivative at x (one tanh).
+__device__ __forceinline__ void gelu_both(float x, float* h, float* g) {
+    const float th = tanhf(kGeluC * (x + kGeluA * x * x * x));
+    *h = 0.5f * x * (1.0f + th);
+    *g = 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluA * x * x);
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    train_kernel(const __half* __restrict__ X, const float* __restrict__ target, const uint32_t* __restrict__ perm,
+                 uint32_t rows, const __half* __restrict__ w1h, const __half* __restrict__ w2h,
+                 const float* __restrict__ params, float inv, GradParts out, unsigned* __restrict__ err) {
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    const uint32_t w1s = base, w2s = base + kOpBytes, xs = base + 2 * kOpBytes, h1s = base + 3 * kOpBytes,
+                   dz2s = base + 4 * kOpBytes, ts = base + 5 * kOpBytes;  // ts: H2, then dZ1
+    float* const b1v = reinterpret_cast<float*>(smem_raw + (base - raw) + 6 * kOpBytes);
+    float *const b2v = b1v + kH, *const w3v = b1v + 2 * kH, *const ysum = b1v + 3 * kH + 4, *const dyv = ysum + 4 * kTileRows;
+    const uint32_t bar = base + 6 * kOpBytes + kTrainFloats * sizeof(float), tmem_slot = bar + 8;
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31, quad = warp & 3, group = warp >> 2;
+    const uint32_t r = quad * 32 + lane, c0 = group * 32;
+    const uint32_t col = t & 127u;  // column sums: this thread's column, over rows c0 .. c0 + 31
+
+    for (uint32_t j = group * 4; j < group * 4 + 4; ++j) {
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        store_chunk(w1s, r, j, r < (uint32_t)kIn ? reinterpret_cast<const uint4*>(w1h + (size_t)r * kH)[j] : zero);
+        store_chunk(w2s, r, j, reinterpret_cast<const uint4*>(w2h + (size_t)r * kH)[j]);
+    }
+    if (t < (uint32_t)kH) {
+        b1v[t] = params[kB1 + t];
+        b2v[t] = params[kB2 + t];
+        w3v[t] = params[kW3 + t];
+    }
+    if (t == 0) {
+        b1v[3 * kH] = params[kB3];
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
+                     "r"(kTrainTmem)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    uint32_t tmem = 0;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
+    const uint32_t z1t = tmem, z2t = tmem + 128, dw2t = tmem + 256, dw1t = tmem + 384;
+    const uint32_t my_lanes = (quad * 32u) << 16;
+    uint32_t phase = 0;
+    bool failed = false, undrained = false;
+    // Issues products from one thread and waits (bounded) for them; all threads call it.
+    auto run = [&](auto issue) {
+        proxy_fence();  // make the operand tiles visible to the tensor cores
+        tc_fence_before();
+        __syncthreads();
+        if (t == 0) {
+            tc_fence_after();
+            issue();
+            umma_commit(bar);
+        }
+        const bool ok = mbar_wait(bar, phase);
+        if (__syncthreads_or(!ok)) {  // timed out: drain the products in flight (bounded), then leave
+            undrained = !__syncthreads_and(mbar_wait(bar, phase));
+            failed = true;
+            return false;
+        }
+        phase ^= 1u;
+        tc_fence_after();
+        return true;
+    };
+
+    float s_w3 = 0.0f, s_b2 = 0.0f, s_b1 = 0.0f, s_b3 = 0.0f, s_loss = 0.0f;
+    for (uint32_t tile = blockIdx.x; (uint64_t)tile * kTileRows < rows; tile += gridDim.x) {
+        const uint32_t i = tile * kTileRows + r;
+        const bool valid = i < rows;
+        const uint32_t src = valid ? (perm ? perm[i] : i) : 0u;
+        const uint4* const xrow = reinterpret_cast<const uint4*>(X + (size_t)src * kIn);
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            const uint32_t j = group * 4 + e;
+            store_chunk(xs, r, j, valid && j < (uint32_t)kIn / 8 ? xrow[j] : make_uint4(0, 0, 0, 0));
+        }
+        const float goal = valid ? target[src] : 0.0f;
+        const uint32_t more = tile != blockIdx.x;  // the weight gradients go on from the tile before
+        if (!run([&] {
+                for (uint32_t k = 0; k < kIn / 16; ++k)
+                    umma_f16(z1t, sw128_desc(xs + kstep_offset(k)), sw128_desc_mn(w1s + k * kKstepRows), k > 0,
+                             kIdesc | kMnB);
+            }))
+            break;
+        float g1[32], g2[32];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            float v[16];
+            tmem_ld16(z1t + my_lanes + c0 + h * 16, v);
+            uint32_t q[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float a, b;
+                gelu_both(v[2 * e] + b1v[c0 + h * 16 + 2 * e], &a, &g1[h * 16 + 2 * e]);
+                gelu_both(v[2 * e + 1] + b1v[c0 + h * 16 + 2 * e + 1], &b, &g1[h * 16 + 2 * e + 1]);
+                q[e] = pack_half2(a, b);
+            }
+            store_chunk(h1s, r, group * 4 + h * 2, make_uint4(q[0], q[1], q[2], q[3]));
+            store_chunk(h1s, r, group * 4 + h * 2 + 1, make_uint4(q[4], q[5], q[6], q[7]));
+        }
+        if (!run([&] {
+                for (uint32_t k = 0; k < 8; ++k)
+                    umma_f16(z2t, sw128_desc(h1s + kstep_offset(k)), sw128_desc_mn(w2s + k * kKstepRows), k > 0,
+                             kIdesc | kMnB);
+            }))
+            break;
+        float y = 0.0f;
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            float v[16];
+            tmem_ld16(z2t + my_lanes + c0 + h * 16, v);
+            uint32_t q[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const uint32_t c = c0 + h * 16 + 2 * e;
+                float a, b;
+                gelu_both(v[2 * e] + b2v[c], &a, &g2[h * 16 + 2 * e]);
+                gelu_both(v[2 * e + 1] + b2v[c + 1], &b, &g2[h * 16 + 2 * e + 1]);
+                q[e] = pack_half2(a, b);
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&q[e]));  // H2 is fp16
+                y += f.x * w3v[c] + f.y * w3v[c + 1];
+            }
+            store_chunk(ts, r, group * 4 + h * 2, make_uint4(q[0], q[1], q[2], q[3]));
+            store_chunk(ts, r, group * 4 + h * 2 + 1, make_uint4(q[4], q[5], q[6], q[7]));
+        }
+        ysum[group * kTileRows + r] = y;
+        __syncthreads();
+        y = ysum[r] + ysum[kTileRows + r] + ysum[2 * kTileRows + r] + ysum[3 * kTileRows + r] + b1v[3 * kH];
+        const float d = valid ? y - goal : 0.0f, dy = 2.0f * d;
+        if (group == 0) {
+            dyv[r] = dy;
+            s_b3 += dy;
+            s_loss += d * d;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            uint32_t q[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t c = e * 8 + 2 * k;
+                q[k] = pack_half2(dy * w3v[c0 + c] * g2[c], dy * w3v[c0 + c + 1] * g2[c + 1]);
+            }
+            store_chunk(dz2s, r, group * 4 + e, make_uint4(q[0], q[1], q[2], q[3]));
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (uint32_t k = c0; k < c0 + 32; ++k) {
+            s_w3 += half_at(ts, k, col) * dyv[k];
+            s_b2 += half_at(dz2s, k, col);
+        }
+        if (!run([&] {
+                for (uint32_t k = 0; k < 8; ++k)
+                    umma_f16(dw2t, sw128_desc_mn(h1s + k * kKstepRows), sw128_desc_mn(dz2s + k * kKstepRows),
+                             more | (k > 0), kIdesc | kMnA | kMnB);
+                for (uint32_t k = 0; k < 8; ++k)
+                    umma_f16(z2t, sw128_desc(dz2s + kstep_offset(k)), sw128_desc(w2s + kstep_offset(k)), k > 0);
+            }))
+            break;
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            float v[16];
+            tmem_ld16(z2t + my_lanes + c0 + h * 16, v);  // dH1
+            uint32_t q[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                q[e] = pack_half2(v[2 * e] * g1[h * 16 + 2 * e], v[2 * e + 1] * g1[h * 16 + 2 * e + 1]);
+            store_chunk(ts, r, group * 4 + h * 2, make_uint4(q[0], q[1], q[2], q[3]));
+            store_chunk(ts, r, group * 4 + h * 2 + 1, make_uint4(q[4], q[5], q[6], q[7]));
+        }
+        if (!run([&] {
+                for (uint32_t k = 0; k < 8; ++k)
+                    umma_f16(dw1t, sw128_desc_mn(xs + k * kKstepRows), sw128_desc_mn(ts + k * kKstepRows),
+                             more | (k > 0), kIdesc | kMnA | kMnB);
+            }))
+            break;
+#pragma unroll 8
+        for (uint32_t k = c0; k < c0 + 32; ++k) s_b1 += half_at(ts, k, col);
+        __syncthreads();  // the row tiles are free for the next 128 rows
+    }
+    if (!failed) {
+        const uint32_t slot = blockIdx.x;
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            float v[16];
+            tmem_ld16(dw2t + my_lanes + c0 + h * 16, v);
+            float4* p = reinterpret_cast<float4*>(out.w2 + (size_t)slot * kH * kH + (size_t)r * kH + c0 + h * 16);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                p[e] = make_float4(inv * v[4 * e], inv * v[4 * e + 1], inv * v[4 * e + 2], inv * v[4 * e + 3]);
+            tmem_ld16(dw1t + my_lanes + c0 + h * 16, v);
+            p = reinterpret_cast<float4*>(out.w1 + (size_t)slot * kW1Size + (size_t)r * kH + c0 + h * 16);
+            if (r < (uint32_t)kIn)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    p[e] = make_float4(inv * v[4 * e], inv * v[4 * e + 1], inv * v[4 * e + 2], inv * v[4 * e + 3]);
+        }
+        // column sums: the four row groups of each column, then b3 and the loss over the rows
+        float* const part = reinterpret_cast<float*>(smem_raw + (base - raw) + 2 * kOpBytes);  // X is free
+        part[t] = s_w3;
+        part[kTrainThreads + t] = s_b2;
+        part[2 * kTrainThreads + t] = s_b1;
+        part[3 * kTrainThreads + t] = s_b3;
+        part[4 * kTrainThreads + t] = s_loss;
+        __syncthreads();
+        if (t < (uint32_t)kH) {
+            auto sum4 = [&](uint32_t k) {
+                const float* p = part + k * kTrainThreads + t;
+                return (p[0] + p[kH]) + (p[2 * kH] + p[3 * kH]);
+            };
+            out.w3[slot * kH + t] = inv * sum4(0);
+            out.b2[slot * kH + t] = inv * sum4(1);
+            out.b1[slot * kH + t] = inv * sum4(2);
+        }
+        if (warp < 2) {  // only the threads of group 0 (t < 128) have summed these
+            const float* p = part + (3 + warp) * kTrainThreads + lane;
+            float v = (p[0] + p[32]) + (p[64] + p[96]);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+            if (lane == 0) out.tail[slot * 2 + warp] = warp == 0 ? inv * v : v;
+        }
+    }
+    // bit 0: a completion wait timed out; bit 1: the drain timed out too, so products may still
+    // have been in flight when the tensor memory was freed
+    if (failed && t == 0) atomicOr(err, undrained ? 3u : 1u);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTrainTmem) : "memory");
+    }
+}
+
+// Gradient of parameter i: the sum over the blocks' slots, in slot order.
+__device__ __forceinline__ float grad_of(const GradParts& g, int i, int slots) {
+    const float* p;
+    size_t stride = kH;
+    if (i < kB1) p = g.w1 + i, stride = kW1Size;
+    else if (i < kW2) p = g.b1 + (i - kB1);
+    else if (i < kB2) p = g.w2 + (i - kW2), stride = kH * kH;
+    else if (i < kW3) p = g.b2 + (i - kB2);
+    else if (i < kB3) p = g.w3 + (i - kW3);
+    else p = g.tail, stride = 2;
+    float s = 0.0f;
+#pragma unroll 8
+    for (int b = 0; b < slots; ++b) s += p[b * stride];
+    return s;
+}
+
+__device__ __forceinline__ void add_loss(const GradParts& g, int slots, float* loss) {
+    float s = 0.0f;
+    for (int b = 0; b < slots; ++b) s += g.tail[2 * b + 1];
+    *loss += s;
+}
+
+__global__ void grad_kernel(GradParts g, int slots, float* __restrict__ out, float* __restrict__ loss,
+                            const unsigned* __restrict__ err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (*err || i >= kParams) return;
+    out[i] = grad_of(g, i, slots);
+    if (i == 0) add_loss(g, slots, loss);
+}
+
+// Adam (Kingma & Ba 2015) on the flat fp32 parameters; refreshes the fp16 copies of W1, W2.
+__global__ void adam_kernel(float* __restrict__ p, GradParts g, int slots, float* __restrict__ m,
+                            float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
+                            __half* __restrict__ w1h, __half* __restrict__ w2h, float* __restrict__ loss,
+                            const unsigned* __restrict__ err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (*err || i >= kParams) return;
+    const float gi = grad_of(g, i, slots);
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float w = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = w;
+    if (i < kW1Size) w1h[i] = __float2half(w);
+    else if (i >= kW2 && i < kB2) w2h[i - kW2] = __float2half(w);
+    if (i == 0) add_loss(g, slots, loss);
+}
+
+// Device buffers of the training steps of one call, for batches of up to `rows` rows.
 struct Work {
-    __half *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
-    float *t = nullptr, *Z = nullptr, *Zb1 = nullptr, *Zb2 = nullptr, *y = nullptr, *dy = nullptr, *dH1 = nullptr,
-          *loss = nullptr;
-    unsigned* err = nullptr;  // set by a GEMM whose tensor-core completion wait timed out
-    uint32_t cap = 0;
+    GradParts parts{};
+    float* loss = nullptr;
+    unsigned* err = nullptr;  // set by a step whose tensor-core completion wait timed out
+    int max_slots = 0;
     cudaStream_t stream;  // the buffers are allocated and freed in its order
     std::vector<void*> owned;
 
@@ -550,38 +628,35 @@ struct Work {
     Work(const Work&) = delete;
     Work& operator=(const Work&) = delete;
 
-    int init(uint32_t rows) {
-        cap = rows;
-        const size_t r = rows;
-        owned.reserve(16);  // may throw, but before anything is allocated; push_back then does not
-        auto get = [&](auto** p, size_t bytes) {
+    int init(uint32_t rows, int device) {
+        int sms = 0, s = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        max_slots = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)rows + kTileRows - 1) / kTileRows, sms));
+        owned.reserve(8);  // may throw, but before anything is allocated; push_back then does not
+        auto get = [&](auto** p, size_t count) {
             void* v = nullptr;
-            const int s = dev_alloc_bytes(&v, bytes, stream);
-            if (s == NQB_OK) {
+            const int st = dev_alloc_bytes(&v, count * sizeof(**p), stream);
+            if (st == NQB_OK) {
                 owned.push_back(v);
                 *p = static_cast<std::remove_pointer_t<decltype(p)>>(v);
             }
-            return s;
+            return st;
         };
-        int s = NQB_OK;
-        if (!s) s = get(&X, r * kIn * sizeof(__half));
-        if (!s) s = get(&H1, r * kH * sizeof(__half));
-        if (!s) s = get(&H2, r * kH * sizeof(__half));
-        if (!s) s = get(&dZ2, r * kH * sizeof(__half));
-        if (!s) s = get(&dZ1, r * kH * sizeof(__half));
-        if (!s) s = get(&t, r * sizeof(float));
-        if (!s) s = get(&Z, r * kH * sizeof(float));
-        if (!s) s = get(&Zb1, r * kH * sizeof(float));
-        if (!s) s = get(&Zb2, r * kH * sizeof(float));
-        if (!s) s = get(&y, r * sizeof(float));
-        if (!s) s = get(&dy, r * sizeof(float));
-        if (!s) s = get(&dH1, r * kH * sizeof(float));
-        if (!s) s = get(&loss, sizeof(float));
-        if (!s) s = get(&err, sizeof(unsigned));
+        const size_t n = max_slots;
+        if (!s) s = get(&parts.w1, n * kW1Size);
+        if (!s) s = get(&parts.b1, n * kH);
+        if (!s) s = get(&parts.w2, n * kH * kH);
+        if (!s) s = get(&parts.b2, n * kH);
+        if (!s) s = get(&parts.w3, n * kH);
+        if (!s) s = get(&parts.tail, n * 2);
+        if (!s) s = get(&loss, 1);
+        if (!s) s = get(&err, 1);
         if (!s) s = cuda_status(cudaMemsetAsync(err, 0, sizeof(unsigned), stream));
+        if (!s)
+            s = cuda_status(cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)kTrainSmem));
         return s;
     }
-    // NQB_E_STALL if a GEMM of the passes so far timed out (synchronises the stream).
+    // NQB_E_STALL if a step so far timed out (synchronises the stream).
     int check(cudaStream_t s) const {
         unsigned h = 0;
         int st = cuda_status(cudaMemcpyAsync(&h, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -615,34 +690,15 @@ namespace nqb {
 namespace mlp {
 namespace {
 
-// Forward and backward over `rows` rows already in w.X / w.t; accumulates the mean
-// squared error into w.loss and writes the mean gradient into m->grad.
-int pass(nqb_model* m, Work& w, uint32_t rows, cudaStream_t s) {
-    const float* P = m->params;
-    float* G = m->grad;
-    int st;
-    cudaMemsetAsync(G, 0, kParams * sizeof(float), s);
-    // forward
-    if ((st = gemm(w.X, kIn, 1, m->w1h, kH, 1, w.Z, kH, rows, kH, kIn, 1.0f, 0.0f, w.err, s))) return st;
-    bias_gelu_kernel<<<blocks_for((uint64_t)rows * kH), 256, 0, s>>>(w.Z, P + kB1, rows, w.Zb1, w.H1);
-    if ((st = gemm(w.H1, kH, 1, m->w2h, kH, 1, w.Z, kH, rows, kH, kH, 1.0f, 0.0f, w.err, s))) return st;
-    bias_gelu_kernel<<<blocks_for((uint64_t)rows * kH), 256, 0, s>>>(w.Z, P + kB2, rows, w.Zb2, w.H2);
-    head_kernel<<<blocks_for((uint64_t)rows * 32), 256, 0, s>>>(w.H2, P + kW3, P + kB3, rows, w.y);
-    loss_kernel<<<blocks_for(rows), 256, 0, s>>>(w.y, w.t, rows, w.dy, w.loss);
-    // backward (mean over the rows)
-    const float inv = 1.0f / (float)rows;
-    colsum_kernel<<<std::min<unsigned>(rows, 512), kH, 0, s>>>(w.H2, w.dy, rows, inv, G + kW3);  // dw3
-    sum_kernel<<<std::min<unsigned>(blocks_for(rows), 256), 256, 0, s>>>(w.dy, rows, inv, G + kB3);
-    dz2_kernel<<<blocks_for((uint64_t)rows * kH), 256, 0, s>>>(w.dy, P + kW3, w.Zb2, rows, w.dZ2);
-    colsum_kernel<<<std::min<unsigned>(rows, 512), kH, 0, s>>>(w.dZ2, nullptr, rows, inv, G + kB2);
-    // dW2 = H1^T dZ2: A(i, k) = H1[k][i], B(k, j) = dZ2[k][j]
-    if ((st = gemm(w.H1, 1, kH, w.dZ2, kH, 1, G + kW2, kH, kH, kH, rows, inv, 0.0f, w.err, s))) return st;
-    // dH1 = dZ2 W2^T: B(k, j) = W2[j][k]
-    if ((st = gemm(w.dZ2, kH, 1, m->w2h, 1, kH, w.dH1, kH, rows, kH, kH, 1.0f, 0.0f, w.err, s))) return st;
-    dz1_kernel<<<blocks_for((uint64_t)rows * kH), 256, 0, s>>>(w.dH1, w.Zb1, rows, w.dZ1);
-    colsum_kernel<<<std::min<unsigned>(rows, 512), kH, 0, s>>>(w.dZ1, nullptr, rows, inv, G + kB1);
-    // dW1 = X^T dZ1
-    if ((st = gemm(w.X, 1, kIn, w.dZ1, kH, 1, G + kW1, kH, kIn, kH, rows, inv, 0.0f, w.err, s))) return st;
+// Forward and backward over `rows` rows (of X and target, through perm when given): the blocks'
+// shares of the mean gradient and of the summed squared error into w.parts.  Returns the
+// number of slots through *slots.
+int pass(const nqb_model* m, Work& w, const __half* X, const float* target, const uint32_t* perm, uint32_t rows,
+         int* slots, cudaStream_t s) {
+    const uint64_t tiles = ((uint64_t)rows + kTileRows - 1) / kTileRows;
+    *slots = (int)std::min<uint64_t>(tiles, (uint64_t)w.max_slots);
+    train_kernel<<<*slots, kTrainThreads, kTrainSmem, s>>>(X, target, perm, rows, m->w1h, m->w2h, m->params,
+                                                           1.0f / (float)rows, w.parts, w.err);
     return cuda_status(cudaGetLastError());
 }
 
@@ -819,15 +875,21 @@ int nqb_model_loss_grad(nqb_model* m, const nqb_state* states, const float* targ
     if (cs.status) return cs.status;
     Work w(cs.s);
     DevBuf<nqb_state> d_st(cs.s);
-    int st = w.init((uint32_t)count);
+    DevBuf<__half> d_X(cs.s);
+    DevBuf<float> d_t(cs.s);
+    int st = w.init((uint32_t)count, m->device);
     if (!st) st = d_st.alloc(count);
+    if (!st) st = d_X.alloc(count * kIn);
+    if (!st) st = d_t.alloc(count);
     if (!st) st = cuda_status(cudaMemcpyAsync(d_st.p, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, cs.s));
-    if (!st) st = cuda_status(cudaMemcpyAsync(w.t, targets, count * sizeof(float), cudaMemcpyHostToDevice, cs.s));
+    if (!st) st = cuda_status(cudaMemcpyAsync(d_t.p, targets, count * sizeof(float), cudaMemcpyHostToDevice, cs.s));
     if (st) return st;
-    features_kernel<<<blocks_for(count * kIn), 256, 0, cs.s>>>(reinterpret_cast<const uint4*>(d_st.p), nullptr,
-                                                                 (uint32_t)count, w.X);
+    features_kernel<<<blocks_for(count * kIn), 256, 0, cs.s>>>(reinterpret_cast<const uint4*>(d_st.p), count, d_X.p);
     cudaMemsetAsync(w.loss, 0, sizeof(float), cs.s);
-    if ((st = pass(m, w, (uint32_t)count, cs.s))) return st;
+    int slots = 0;
+    if ((st = pass(m, w, d_X.p, d_t.p, nullptr, (uint32_t)count, &slots, cs.s))) return st;
+    grad_kernel<<<blocks_for(kParams), 256, 0, cs.s>>>(w.parts, slots, m->grad, w.loss, w.err);
+    if ((st = cuda_status(cudaGetLastError()))) return st;
     float l = 0;
     st = cuda_status(cudaMemcpyAsync(&l, w.loss, sizeof(float), cudaMemcpyDeviceToHost, cs.s));
     if (!st) st = cuda_status(cudaMemcpyAsync(grad, m->grad, kParams * sizeof(float), cudaMemcpyDeviceToHost, cs.s));
@@ -856,7 +918,7 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
     DevBuf<__half> d_X(cs.s);
     DevBuf<float> d_t(cs.s);
     DevBuf<uint32_t> d_perm(cs.s);
-    int st = w.init(B);
+    int st = w.init(B, m->device);
     if (!st) st = d_st.alloc(count);
     if (!st) st = d_X.alloc(count * kIn);
     if (!st) st = d_t.alloc(count);
@@ -864,8 +926,7 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
     if (!st) st = cuda_status(cudaMemcpyAsync(d_st.p, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, cs.s));
     if (!st) st = cuda_status(cudaMemcpyAsync(d_t.p, targets, count * sizeof(float), cudaMemcpyHostToDevice, cs.s));
     if (st) return st;
-    features_kernel<<<blocks_for(count * kIn), 256, 0, cs.s>>>(reinterpret_cast<const uint4*>(d_st.p), nullptr,
-                                                                 (uint32_t)count, d_X.p);
+    features_kernel<<<blocks_for(count * kIn), 256, 0, cs.s>>>(reinterpret_cast<const uint4*>(d_st.p), count, d_X.p);
     std::vector<uint32_t> perm(count);
     for (uint64_t i = 0; i < count; ++i) perm[i] = (uint32_t)i;
     uint64_t rng = o.seed * 0x9E3779B97F4A7C15ull + 1;
@@ -876,21 +937,24 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
         return z ^ (z >> 31);
     };
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    for (int ep = 0; ep < o.epochs; ++ep) {
+    auto shuffle = [&] {
         for (uint64_t i = count - 1; i > 0; --i) std::swap(perm[i], perm[next() % (i + 1)]);  // Fisher-Yates
+    };
+    shuffle();
+    for (int ep = 0; ep < o.epochs; ++ep) {
         st = cuda_status(cudaMemcpyAsync(d_perm.p, perm.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, cs.s));
         if (st) return st;
         cudaMemsetAsync(w.loss, 0, sizeof(float), cs.s);
         for (uint64_t off = 0; off < count; off += B) {
             const uint32_t rows = (uint32_t)std::min<uint64_t>(B, count - off);
-            gather_f16_rows<<<blocks_for((uint64_t)rows * kIn), 256, 0, cs.s>>>(d_X.p, d_perm.p + off, rows, w.X);
-            gather_f32<<<blocks_for(rows), 256, 0, cs.s>>>(d_t.p, d_perm.p + off, rows, w.t);
-            if ((st = pass(m, w, rows, cs.s))) return st;
+            int slots = 0;
+            if ((st = pass(m, w, d_X.p, d_t.p, d_perm.p + off, rows, &slots, cs.s))) return st;
             m->adam_step++;
             const float c1 = 1.0f - std::pow(b1, (float)m->adam_step), c2 = 1.0f - std::pow(b2, (float)m->adam_step);
-            adam_kernel<<<blocks_for(kParams), 256, 0, cs.s>>>(m->params, m->grad, m->m, m->v, kParams, o.lr, b1, b2,
-                                                                eps, c1, c2, m->w1h, m->w2h);
+            adam_kernel<<<blocks_for(kParams), 256, 0, cs.s>>>(m->params, w.parts, slots, m->m, m->v, o.lr, b1, b2, eps,
+                                                                c1, c2, m->w1h, m->w2h, w.loss, w.err);
         }
+        if (ep + 1 < o.epochs) shuffle();  // the next epoch's order, while the device works on this one
         float l = 0;
         st = cuda_status(cudaMemcpyAsync(&l, w.loss, sizeof(float), cudaMemcpyDeviceToHost, cs.s));
         if (!st) st = w.check(cs.s);
