@@ -40,7 +40,6 @@ constexpr uint32_t kSpinLimit = 1u << 22;  // waits: far above the ~1 us a produ
 // instruction descriptor, kind::f16: D fp32 (bits 4-5 = 1), A and B fp16 and K-major,
 // N >> 3 at bits 17-22, M >> 4 at bits 24-28
 constexpr uint32_t kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr size_t kPredictSmem = 1024 /* alignment slack */ + 3 * kOpBytes + (3 * kH + 4) * sizeof(float) + 16;
 
 __device__ __forceinline__ uint32_t sw128_chunk(uint32_t r, uint32_t j) {
     return (j >> 3) * kAtomBytes + r * 128u + (((j & 7u) ^ (r & 7u)) << 4);
@@ -143,54 +142,59 @@ __global__ void to_half_kernel(const float* __restrict__ p, __half* __restrict__
     if (i < kH * kH) w2h[i] = __float2half(p[kW2 + i]);
 }
 
-// ---- fused inference on the 5th-generation tensor cores (tcgen05) ----------------------
-// One CTA of 4 warps runs 128-row tiles: features -> layer 1 -> GELU -> layer 2 -> GELU ->
-// head.  Both layers are M=128, N=128, K=128 products (the 112 inputs zero-padded) issued as
-// eight K=16 tcgen05.mma by one thread, with FP16 operands in shared memory and the FP32
-// accumulator in tensor memory (128 lanes x 128 columns).  Thread t owns tile row t: it
-// builds that row's features, and after each layer reads the row's 128 accumulators with
-// tcgen05.ld (warp w may read lanes 32w..32w+31), so GELU and the head's dot product need
-// no shuffles.  Operand tiles use the 128-byte-swizzled K-major layout: 16-byte chunk j of
-// row r of a 128-row tile sits at (j / 8) x 16 KB + r x 128 + ((j % 8) ^ (r % 8)) x 16.
-// Every wait on the MMA completion barrier is bounded; on a timeout the block sets the
-// error word and leaves, freeing its tensor memory on the way out.
-// Writes W (math layout [in][out], fp16, `in_rows` real inputs) as the B operand: tile row n
-// = output n, K = input, zero beyond in_rows.  Thread t writes row t.
-__device__ __forceinline__ void stage_weights(uint32_t tile, const __half* __restrict__ w, int in_rows, uint32_t t) {
-    for (uint32_t j = 0; j < 16; ++j) {
-        uint32_t q[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k0 = (int)j * 8 + 2 * e;
-            const float a = k0 < in_rows ? __half2float(w[(size_t)k0 * kH + t]) : 0.0f;
-            const float b = k0 + 1 < in_rows ? __half2float(w[(size_t)(k0 + 1) * kH + t]) : 0.0f;
-            q[e] = pack_half2(a, b);
-        }
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + sw128_chunk(t, j)), "r"(q[0]), "r"(q[1]),
-                     "r"(q[2]), "r"(q[3])
-                     : "memory");
-    }
+__device__ __forceinline__ void store_chunk(uint32_t tile, uint32_t r, uint32_t j, uint4 q) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + sw128_chunk(r, j)), "r"(q.x), "r"(q.y),
+                 "r"(q.z), "r"(q.w)
+                 : "memory");
 }
 
-__global__ void __launch_bounds__(128) predict_kernel(const uint4* __restrict__ st, uint32_t count,
-                                                      const __half* __restrict__ w1h, const __half* __restrict__ w2h,
-                                                      const float* __restrict__ params, float* __restrict__ out,
-                                                      uint32_t wait_limit, unsigned* __restrict__ err) {
+// Features 8 j .. 8 j + 7 of a state as four fp16 pairs.
+__device__ __forceinline__ void feature_chunk(const uint4 s, uint32_t j, uint32_t q[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) q[e] = pack_half2(feature(s, (int)j * 8 + 2 * e), feature(s, (int)j * 8 + 2 * e + 1));
+}
+
+// ---- fused inference (tcgen05) ----------------------------------------------------------------
+// A block of 16 warps runs 128-row tiles: features -> layer 1 -> GELU -> layer 2 -> GELU -> head.
+// Both layers are M=128, N=128 products (K = 112 and 128) issued as K=16 tcgen05.mma by one
+// thread, with FP16 operands in shared memory and the FP32 accumulator in tensor memory.
+// Threads share the work as in train_kernel: row 32 quad + lane, hidden columns (and feature
+// columns) 32 group .. 32 group + 31; the head's four partial sums of a row meet in shared
+// memory.  H1 replaces the features in the row tile.  Every wait on the MMA completion barrier
+// is bounded; on a timeout the block sets the error word and leaves, freeing its tensor memory
+// on the way out.
+//
+// What bounds it: the tanh of 256 activations and the features of each row, and the waits of a
+// tile's chain; two blocks an SM take turns at it.  300,000 rows: 119 us
+// (190 us with 4 warps a block, each thread a whole row).
+constexpr uint32_t kPredictThreads = 512;
+constexpr uint32_t kPredictFloats = 3 * kH + 4 + 4 * kTileRows;  // b1 b2 w3 b3 | y partials
+constexpr size_t kPredictSmem = 1024 /* alignment slack */ + 3 * kOpBytes + kPredictFloats * sizeof(float) + 16;
+
+__global__ void __launch_bounds__(kPredictThreads, 2)
+    predict_kernel(const uint4* __restrict__ st, uint32_t count, const __half* __restrict__ w1h,
+                   const __half* __restrict__ w2h, const float* __restrict__ params, float* __restrict__ out,
+                   uint32_t wait_limit, unsigned* __restrict__ err) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
     const uint32_t w1s = base, w2s = base + kOpBytes, xs = base + 2 * kOpBytes;
-    float* vec = reinterpret_cast<float*>(smem_raw + (base - raw) + 3 * kOpBytes);  // b1 | b2 | w3 | b3
-    const uint32_t bar = base + 3 * kOpBytes + (3 * kH + 4) * sizeof(float);
+    float* const vec = reinterpret_cast<float*>(smem_raw + (base - raw) + 3 * kOpBytes);  // b1 | b2 | w3 | b3
+    float* const ysum = vec + 3 * kH + 4;
+    const uint32_t bar = base + 3 * kOpBytes + kPredictFloats * sizeof(float);
     const uint32_t tmem_slot = bar + 8;
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31, quad = warp & 3, group = warp >> 2;
+    const uint32_t r = quad * 32 + lane, c0 = group * 32;
 
-    stage_weights(w1s, w1h, kIn, t);
-    stage_weights(w2s, w2h, kH, t);
-    for (uint32_t e = t; e < (uint32_t)kH; e += blockDim.x) {
-        vec[e] = params[kB1 + e];
-        vec[kH + e] = params[kB2 + e];
-        vec[2 * kH + e] = params[kW3 + e];
+    for (uint32_t j = group * 4; j < group * 4 + 4; ++j) {
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        store_chunk(w1s, r, j, r < (uint32_t)kIn ? reinterpret_cast<const uint4*>(w1h + (size_t)r * kH)[j] : zero);
+        store_chunk(w2s, r, j, reinterpret_cast<const uint4*>(w2h + (size_t)r * kH)[j]);
+    }
+    if (t < (uint32_t)kH) {
+        vec[t] = params[kB1 + t];
+        vec[kH + t] = params[kB2 + t];
+        vec[2 * kH + t] = params[kW3 + t];
     }
     if (t == 0) {
         vec[3 * kH] = params[kB3];
@@ -203,29 +207,24 @@ __global__ void __launch_bounds__(128) predict_kernel(const uint4* __restrict__ 
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    proxy_fence();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     uint32_t tmem = 0;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
-    const uint32_t my_lanes = tmem + ((warp * 32u) << 16);
+    const uint32_t mine = tmem + ((quad * 32u) << 16) + c0;
     uint32_t phase = 0;
     bool failed = false, undrained = false;
 
     for (uint32_t tile = blockIdx.x; (uint64_t)tile * kTileRows < count && !failed; tile += gridDim.x) {
-        const uint64_t i = (uint64_t)tile * kTileRows + t;
+        const uint64_t i = (uint64_t)tile * kTileRows + r;
         const uint4 s = i < count ? st[i] : make_uint4(0, 0, 0, 0);
-        for (uint32_t j = 0; j < 16; ++j) {  // the row's 128 features (zero for rows past the end)
-            uint32_t q[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int k0 = (int)j * 8 + 2 * e;
-                q[e] = i < count ? pack_half2(feature(s, k0), feature(s, k0 + 1)) : 0u;
-            }
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(xs + sw128_chunk(t, j)), "r"(q[0]),
-                         "r"(q[1]), "r"(q[2]), "r"(q[3])
-                         : "memory");
+#pragma unroll 1
+        for (uint32_t e = 0; e < 4; ++e) {  // 32 of the row's features (zero for rows past the end)
+            const uint32_t j = group * 4 + e;
+            uint32_t q[4] = {0u, 0u, 0u, 0u};
+            if (i < count) feature_chunk(s, j, q);
+            store_chunk(xs, r, j, make_uint4(q[0], q[1], q[2], q[3]));
         }
         float sum = 0.0f;
         for (int layer = 0; layer < 2 && !failed; ++layer) {
@@ -235,9 +234,10 @@ __global__ void __launch_bounds__(128) predict_kernel(const uint4* __restrict__ 
             if (t == 0) {
                 tc_fence_after();
                 const uint32_t wt = layer == 0 ? w1s : w2s;
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    umma_f16(tmem, sw128_desc(xs + kstep_offset(k)), sw128_desc(wt + kstep_offset(k)), k > 0 ? 1u : 0u);
+                const int steps = layer == 0 ? kIn / 16 : kH / 16;
+                for (int k = 0; k < steps; ++k)
+                    umma_f16(tmem, sw128_desc(xs + kstep_offset(k)), sw128_desc_mn(wt + k * kKstepRows), k > 0 ? 1u : 0u,
+                             kIdesc | kMnB);
                 umma_commit(bar);
             }
             const bool ok = wait_limit ? mbar_wait(bar, phase, wait_limit, true) : mbar_wait(bar, phase);
@@ -248,31 +248,36 @@ __global__ void __launch_bounds__(128) predict_kernel(const uint4* __restrict__ 
             }
             phase ^= 1u;
             tc_fence_after();
-            const float* bias = vec + layer * kH;
-            for (uint32_t c = 0; c < (uint32_t)kH; c += 16) {
-                float v[16];
-                tmem_ld16(my_lanes + c, v);
-                if (layer == 0) {  // H1 = gelu(Z1 + b1), fp16, becomes the A operand of layer 2
-                    uint32_t q[8];
+            const float* bias = vec + layer * kH + c0;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        q[e] = pack_half2(gelu(v[2 * e] + bias[c + 2 * e]), gelu(v[2 * e + 1] + bias[c + 2 * e + 1]));
-                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(xs + sw128_chunk(t, c / 8)),
-                                 "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3])
-                                 : "memory");
-                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(xs + sw128_chunk(t, c / 8 + 1)),
-                                 "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7])
-                                 : "memory");
+            for (uint32_t h = 0; h < 2; ++h) {
+                float v[16];
+                tmem_ld16(mine + h * 16, v);
+                uint32_t q[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    q[e] = pack_half2(gelu(v[2 * e] + bias[h * 16 + 2 * e]),
+                                      gelu(v[2 * e + 1] + bias[h * 16 + 2 * e + 1]));
+                if (layer == 0) {  // H1 becomes the A operand of layer 2
+                    store_chunk(xs, r, group * 4 + h * 2, make_uint4(q[0], q[1], q[2], q[3]));
+                    store_chunk(xs, r, group * 4 + h * 2 + 1, make_uint4(q[4], q[5], q[6], q[7]));
                 } else {  // head: H2 rounded to fp16 as in the training forward pass
 #pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        sum += __half2float(__float2half(gelu(v[e] + bias[c + e]))) * vec[2 * kH + c + e];
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&q[e]));
+                        const float* w3 = vec + 2 * kH + c0 + h * 16 + 2 * e;
+                        sum += f.x * w3[0] + f.y * w3[1];
+                    }
                 }
             }
             tc_fence_before();
         }
-        if (!failed && i < count) out[i] = sum + vec[3 * kH];
-        __syncthreads();  // the operand tile and the accumulator are free for the next tile
+        if (!failed) {
+            ysum[group * kTileRows + r] = sum;
+            __syncthreads();  // also: the operand tile and the accumulator are free for the next tile
+            if (group == 0 && i < count)
+                out[i] = ysum[r] + ysum[kTileRows + r] + ysum[2 * kTileRows + r] + ysum[3 * kTileRows + r] + vec[3 * kH];
+        }
     }
     // bit 0: a completion wait timed out; bit 1: the drain timed out too, so products may still
     // have been in flight when the tensor memory was freed
@@ -317,12 +322,6 @@ __device__ __forceinline__ float half_at(uint32_t tile, uint32_t r, uint32_t c) 
     unsigned short h;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(tile + sw128_chunk(r, c >> 3) + (c & 7u) * 2u));
     return __half2float(__ushort_as_half(h));
-}
-
-__device__ __forceinline__ void store_chunk(uint32_t tile, uint32_t r, uint32_t j, uint4 q) {
-    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + sw128_chunk(r, j)), "r"(q.x), "r"(q.y),
-                 "r"(q.z), "r"(q.w)
-                 : "memory");
 }
 
 // gelu and its derivative at x (one tanh).
@@ -975,7 +974,7 @@ int model_predict_device(const nqb_model* m, const nqb_state* d_states, uint32_t
     if (e != cudaSuccess) return cuda_status(e);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    const uint64_t tiles = (count + kTileRows - 1) / kTileRows;
+    const uint64_t tiles = ((uint64_t)count + kTileRows - 1) / kTileRows;
     // at most 2 blocks per SM (shared memory), so their tensor memory (2 x 128 columns) fits
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)sms * 2));
     unsigned* d_err = nullptr;
@@ -983,8 +982,8 @@ int model_predict_device(const nqb_model* m, const nqb_state* d_states, uint32_t
     unsigned h_err = 0;
     int st = cuda_status(cudaMemsetAsync(d_err, 0, sizeof(unsigned), s));
     if (!st) {
-        predict_kernel<<<grid, kTileRows, kPredictSmem, s>>>(reinterpret_cast<const uint4*>(d_states), count, m->w1h,
-                                                             m->w2h, m->params, d_out, wait_limit, d_err);
+        predict_kernel<<<grid, kPredictThreads, kPredictSmem, s>>>(reinterpret_cast<const uint4*>(d_states), count,
+                                                                   m->w1h, m->w2h, m->params, d_out, wait_limit, d_err);
         st = cuda_status(cudaGetLastError());
     }
     if (!st) st = cuda_status(cudaMemcpyAsync(&h_err, d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
