@@ -162,7 +162,7 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
         sched.items = own.n;
         if (batched)
             NQB_TRY(launch_batched(own.items, own.n, nullptr, nullptr, d_out + 8, kBatchedScratchBytes, d_out, nullptr,
-                                   nullptr, o.block_size, own.stack_depth, sc.device, sc.stream, &launches, d_lanes));
+                                   nullptr, o.block_size, own.stack_depth, sc.device, sc.stream, &launches, d_lanes, 0, true));
         else
             NQB_TRY(launch_plain(own.items, own.n, d_out, nullptr, o.block_size, o.count_unit_nodes != 0,
                                  own.stack_depth, sc.stream, &launches, d_lanes));

@@ -76,12 +76,13 @@ uint32_t batched_ring_slots(size_t scratch_bytes);
 // d_order (optional): queue position -> item; d_board_of (optional): item -> output slot.
 // d_out: {weighted count, nodes, 0, error flags}.  d_lane_stats as for launch_plain.
 // wait_limit: polls without progress before a wait of the work stealing gives up (0 =
-// kBatchedWaitLimit).
+// kBatchedWaitLimit).  refined: the items have been through refine_items, so few of them means
+// little work.
 int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d_order, const uint32_t* d_board_of,
                    void* d_scratch, size_t scratch_bytes, unsigned long long* d_out,
                    unsigned long long* d_per_board, unsigned long long* d_per_board_nodes, int block_size,
                    unsigned stack_depth, int device, cudaStream_t stream, unsigned* launches,
-                   unsigned long long* d_lane_stats = nullptr, uint32_t wait_limit = 0);
+                   unsigned long long* d_lane_stats = nullptr, uint32_t wait_limit = 0, bool refined = false);
 
 // Items split until a launch has several a lane (refine.cu): the caller's arrays, or device
 // copies owned until release() (a stream-ordered free).  Placements of split items are added

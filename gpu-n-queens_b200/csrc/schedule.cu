@@ -268,7 +268,8 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
                               d_out, d_per_board_nodes, launches, &r);
         if (!st)
             st = launch_batched(r.items, r.n, nullptr, r.board, d_scratch, scratch_bytes, d_out, d_per_board,
-                                d_per_board_nodes, o.block_size, r.stack_depth, device, s, launches, d_lane_stats);
+                                d_per_board_nodes, o.block_size, r.stack_depth, device, s, launches, d_lane_stats, 0,
+                                true);
         r.release();  // stream-ordered after the kernel that reads the arrays
         if (info) info->items = r.n;
         return st;
