@@ -141,40 +141,40 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     unsigned launches = 0;
     SchedInfo sched;
     Refined own;
+    const ItemLevel* d_levels = nullptr;  // a pool's, or the one level of deferred items
+    unsigned n_levels = 0;
+    cudaEvent_t e0 = nullptr;
     if (pool) {
-        cudaEvent_t e0;
         NQB_TRY(sc.event(&e0));
         NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
         const int s = small_pool_items(pool->n, pool->depth, o.count_unit_nodes && !batched, sc.device, sc.stream,
-                                       d_out, &launches, &own, &count);
+                                       d_out, &launches, &own, &d_levels, &n_levels);
         sc.hold(own.buf);
         NQB_TRY(s);
         NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
-        float g = 0.0f;
-        cudaEventSynchronize(e1);
-        cudaEventElapsedTime(&g, e0, e1);
-        pool->gen_ms = g;
-    } else {
-        NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
-    }
-    sched.items = count;
-    if (pool) {
         sched.items = own.n;
         if (batched)
             NQB_TRY(launch_batched(own.items, own.n, nullptr, nullptr, d_out + 8, kBatchedScratchBytes, d_out, nullptr,
-                                   nullptr, o.block_size, own.stack_depth, sc.device, sc.stream, &launches, d_lanes, 0, true));
+                                   nullptr, o.block_size, own.stack_depth, sc.device, sc.stream, &launches, d_lanes, 0,
+                                   true, own.level));
         else
             NQB_TRY(launch_plain(own.items, own.n, d_out, nullptr, o.block_size, o.count_unit_nodes != 0,
-                                 own.stack_depth, sc.stream, &launches, d_lanes));
-    } else if (count) {
-        if (batched) {
-            NQB_TRY(launch_batched_scheduled(d_states, (uint32_t)count, nullptr, d_out + 8, kBatchedScratchBytes, d_out,
-                                             d_per, d_per_nodes, o, depth, sc.device, sc.stream, &launches, &sched,
-                                             d_lanes));
-        } else {
-            NQB_TRY(launch_plain_refined(d_states, count, d_out, d_per, o, depth, sc.device, sc.stream, &launches,
-                                         &sched, d_lanes));
-        }
+                                 own.stack_depth, sc.stream, &launches, d_lanes, nullptr, own.level));
+    } else {
+        NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
+        sched.items = count;
+        int s = NQB_OK;
+        if (count && batched)
+            s = launch_batched_scheduled(d_states, (uint32_t)count, nullptr, d_out + 8, kBatchedScratchBytes, d_out,
+                                         d_per, d_per_nodes, o, depth, sc.device, sc.stream, &launches, &sched,
+                                         d_lanes, &own);
+        else if (count)
+            s = launch_plain_refined(d_states, count, d_out, d_per, o, depth, sc.device, sc.stream, &launches, &sched,
+                                     d_lanes, &own);
+        sc.hold(own.buf);
+        NQB_TRY(s);
+        d_levels = own.level;
+        n_levels = own.level ? 1 : 0;
     }
     NQB_TRY(cuda_status(cudaEventRecord(e2, sc.stream)));
     unsigned long long lanes[2] = {0, 0};
@@ -188,7 +188,19 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     if (per_state_nodes)
         NQB_TRY(cuda_status(cudaMemcpyAsync(per_state_nodes, d_per_nodes, count * sizeof(unsigned long long),
                                             cudaMemcpyDeviceToHost, sc.stream)));
+    ItemLevel levels[kMaxItemLevels];
+    if (n_levels)
+        NQB_TRY(cuda_status(cudaMemcpyAsync(levels, d_levels, n_levels * sizeof(ItemLevel), cudaMemcpyDeviceToHost,
+                                            sc.stream)));
     NQB_TRY(cuda_status(cudaStreamSynchronize(sc.stream)));
+    if (n_levels) sched.items = levels[n_levels - 1].n;
+    if (pool) {
+        if (levels[pool->depth - 1].done != pool->depth - 1) return NQB_E_RANGE;
+        count = levels[pool->depth - 1].n;
+        float g = 0.0f;
+        cudaEventElapsedTime(&g, e0, e1);
+        pool->gen_ms = g;
+    }
     if (totals[3] & 4) return NQB_E_STALL;
     if (totals[3]) return NQB_E_DEVICE;
     if (st) {

@@ -82,6 +82,7 @@ struct BatchArgs {
     const uint32_t* order;     // optional: queue position -> item index
     const uint32_t* board_of;  // optional: item index -> output slot (default: item index)
     uint32_t n_items;
+    const ItemLevel* level;    // SPREAD, optional: items, board_of and n_items are read here instead
     uint32_t stack_depth;
     uint32_t* ctl;                        // zero at launch: item head, hungry warps, ring head, ring tail,
                                           // started warps
@@ -185,8 +186,9 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
     // SPREAD (launches with fewer items than lanes): a refill claims only the warp's share of
     // the items, so they spread over every warp before any splitting starts.  A separate
     // instance: the same few instructions cost the large launches 2.5% (measured at N=21).
+    const uint32_t warps = gridDim.x * (BLOCK / 32);
     const uint32_t claim_cap =
-        SPREAD ? max(1u, (a.n_items + gridDim.x * (BLOCK / 32) - 1) / (gridDim.x * (BLOCK / 32))) : 0u;
+        SPREAD ? max(1u, ((a.level ? a.level->n : a.n_items) + warps - 1) / warps) : 0u;
 
     for (;;) {
         const bool me_idle = s.avail == 0 && s.sp == base;
@@ -198,7 +200,8 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
                 const unsigned long long c = piece_sols * weight;
                 total += c;
                 total_nodes += piece_nodes;
-                const uint32_t slot = a.board_of ? __ldg(a.board_of + item) : item;
+                const uint32_t* const board_of = SPREAD && a.level ? a.level->board : a.board_of;
+                const uint32_t slot = board_of ? __ldg(board_of + item) : item;
                 if (a.per_board && c) atomicAdd(a.per_board + slot, c);
                 if (a.per_board_nodes && piece_nodes) atomicAdd(a.per_board_nodes + slot, piece_nodes);
                 item = kNoItem;
@@ -210,12 +213,13 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
                 uint32_t start = 0;
                 if (lane == 0) start = atomicAdd(a.ctl, k);
                 start = __shfl_sync(kFull, start, 0);
-                if (start + k >= a.n_items) qempty = true;
+                const uint32_t n_items = SPREAD && a.level ? a.level->n : a.n_items;
+                if (start + k >= n_items) qempty = true;
                 const uint32_t ri = __popc(idle & lt_mask);
                 const uint32_t q = start + ri;
-                if (me_idle && (!SPREAD || ri < k) && q < a.n_items) {
+                if (me_idle && (!SPREAD || ri < k) && q < n_items) {
                     const uint32_t it = a.order ? __ldg(a.order + q) : q;
-                    const uint4 st = __ldg(a.items + it);
+                    const uint4 st = __ldg((SPREAD && a.level ? a.level->items : a.items) + it);
                     base = base0;
                     write_sentinel(base0);
                     if (lane_load(s, st, base) > a.stack_depth) {
@@ -398,7 +402,8 @@ int launch_batched_t(BatchArgs a, bool refined, int device, cudaStream_t stream,
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(wave, most));
     const uint64_t lanes = (uint64_t)grid * BLOCK;
     a.donate_every = a.n_items >= kPlentyItems * lanes ? kDonateEveryPlenty : kDonateEvery;
-    if (a.ring_cap && !refined && a.n_items < lanes)
+    // (the large launches' instance reads no level: the branch in their loop cost 0.4%)
+    if (a.level || (a.ring_cap && !refined && a.n_items < lanes))
         spread<<<grid, BLOCK, smem, stream>>>(a);
     else
         kern<<<grid, BLOCK, smem, stream>>>(a);
@@ -422,8 +427,9 @@ int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d
                    void* d_scratch, size_t scratch_bytes, unsigned long long* d_out,
                    unsigned long long* d_per_board, unsigned long long* d_per_board_nodes, int block_size,
                    unsigned stack_depth, int device, cudaStream_t stream, unsigned* launches,
-                   unsigned long long* d_lane_stats, uint32_t wait_limit, bool refined) {
-    if (!d_out || !d_scratch || scratch_bytes < sizeof(uint32_t) || (n_items && !d_items)) return NQB_E_INVALID;
+                   unsigned long long* d_lane_stats, uint32_t wait_limit, bool refined,
+                   const ItemLevel* d_level) {
+    if (!d_out || !d_scratch || scratch_bytes < sizeof(uint32_t) || (n_items && !d_items && !d_level)) return NQB_E_INVALID;
     if (n_items == 0) return NQB_OK;
     if (n_items > (1u << 31)) return NQB_E_RANGE;
     if (stack_depth == 0) stack_depth = NQB_MAX_N - 1;
@@ -436,6 +442,7 @@ int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d
     a.order = d_order;
     a.board_of = d_board_of;
     a.n_items = n_items;
+    a.level = d_level;
     a.stack_depth = stack_depth;
     a.ctl = static_cast<uint32_t*>(d_scratch);
     a.ring_cap = batched_ring_slots(scratch_bytes);

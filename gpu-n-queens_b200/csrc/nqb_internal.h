@@ -52,14 +52,25 @@ unsigned host_threads();
 // pending alternatives one search can hold.
 unsigned max_stack_depth(const nqb_state* states, uint64_t count);
 
+// The items of one level of a split (refine.cu), in device memory.
+struct ItemLevel {
+    const uint4* items;
+    const uint32_t* board;    // item -> output slot (nullptr: identity)
+    unsigned long long next;  // items the next level would make of these
+    uint32_t n;
+    uint32_t done;            // levels that split something
+};
+
 // Plain search kernel (plain.cu).  d_out: {weighted count, nodes, unit nodes, error flags}.
 // d_per_state (optional, zero at launch): weight x completions per state.  d_lane_stats (optional): the
 // instrumented kernel adds {lane-steps that placed a queen, lane-step slots} into it.
-// d_board_of (optional): state -> slot of d_per_state.
+// d_board_of (optional): state -> slot of d_per_state.  d_level (optional, device memory): the
+// states, their number and their slots are read there when the kernel runs, and `count` is only
+// the number expected.
 int launch_plain(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
                  unsigned long long* d_per_state, int block_size, bool count_unit, unsigned stack_depth,
                  cudaStream_t stream, unsigned* launches, unsigned long long* d_lane_stats = nullptr,
-                 const uint32_t* d_board_of = nullptr);
+                 const uint32_t* d_board_of = nullptr, const ItemLevel* d_level = nullptr);
 
 // Scratch of one batched launch (zeroed before it): 64 bytes of control words (word 0 is
 // the item queue head), then the steal ring, 32 bytes a slot.  Scratch of 4 bytes (the
@@ -77,37 +88,42 @@ uint32_t batched_ring_slots(size_t scratch_bytes);
 // d_out: {weighted count, nodes, 0, error flags}.  d_lane_stats as for launch_plain.
 // wait_limit: polls without progress before a wait of the work stealing gives up (0 =
 // kBatchedWaitLimit).  refined: the items have been through refine_items, so few of them means
-// little work.
+// little work.  d_level as for launch_plain.
 int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d_order, const uint32_t* d_board_of,
                    void* d_scratch, size_t scratch_bytes, unsigned long long* d_out,
                    unsigned long long* d_per_board, unsigned long long* d_per_board_nodes, int block_size,
                    unsigned stack_depth, int device, cudaStream_t stream, unsigned* launches,
-                   unsigned long long* d_lane_stats = nullptr, uint32_t wait_limit = 0, bool refined = false);
+                   unsigned long long* d_lane_stats = nullptr, uint32_t wait_limit = 0, bool refined = false,
+                   const ItemLevel* d_level = nullptr);
 
 // Items split until a launch has several a lane (refine.cu): the caller's arrays, or device
 // copies owned until release() (a stream-ordered free).  Placements of split items are added
 // into d_totals[1] (unit: the unit ones also into d_totals[2]) and d_board_nodes[board].
-// boards: the items' output slots are needed.  Waits for the stream when it splits.
+// boards: the items' output slots are needed.  Waits for the stream when it splits, unless
+// may_defer and the items are small: `level` then holds the items and n the number expected.
 struct Refined {
     const nqb_state* items = nullptr;
     const uint32_t* board = nullptr;  // item -> output slot (nullptr: identity)
     uint32_t n = 0;
     unsigned stack_depth = 0;         // bound of the items as they are now
+    const ItemLevel* level = nullptr; // device memory; set when the host has not waited
     void* buf = nullptr;
     cudaStream_t stream = nullptr;
     void release();
 };
 int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, bool boards, bool unit,
                  unsigned stack_depth, int device, cudaStream_t s, unsigned long long* d_totals,
-                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out);
+                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out, bool may_defer = false);
 
 // The (n, depth) pool of a count, split further when it is small, without reading any level's
 // size back: for pools of which small_pool(n, depth) says that they fit refine_items' buffers.
-// *states is the pool's size, `out` the items to search (in no particular order).  Counts like
-// refine_items.  NQB_E_RANGE: the pool did not fit after all.
+// `out` holds the items to search, in no particular order; counts like refine_items, and defers
+// like it.  *levels (device memory, *n_levels of them): every level from the seeds on; the pool is
+// levels[depth - 1], and did not fit after all unless its `done` is depth - 1.
 bool small_pool(unsigned n, unsigned depth);
+constexpr unsigned kMaxItemLevels = NQB_MAX_N + 4;
 int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
-                     unsigned* launches, Refined* out, uint64_t* states);
+                     unsigned* launches, Refined* out, const ItemLevel** levels, unsigned* n_levels);
 
 // Items after learned scheduling: the caller's arrays, or split / ordered device copies
 // owned by the schedule until release() (stream-ordered frees).
@@ -132,7 +148,8 @@ int schedule_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board
 
 // Batched form with optional learned scheduling (schedule.cu): with o.model, items are
 // split and ordered by predicted cost before the launch; otherwise few items are split
-// (refine.cu) and the queue keeps no order.
+// (refine.cu) and the queue keeps no order.  keep (optional): takes the split items over, which
+// may then be deferred (Refined::level).
 struct SchedInfo {
     uint64_t items = 0;     // items given to the search kernel
     double sched_ms = 0.0;  // prediction + splitting + ordering (device time)
@@ -141,13 +158,13 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
                              size_t scratch_bytes, unsigned long long* d_out, unsigned long long* d_per_board,
                              unsigned long long* d_per_board_nodes, const nqb_opts& o, unsigned stack_depth,
                              int device, cudaStream_t s, unsigned* launches, SchedInfo* info,
-                             unsigned long long* d_lane_stats = nullptr);
+                             unsigned long long* d_lane_stats = nullptr, Refined* keep = nullptr);
 
 // Plain form of the library's own calls: few items are split first (refine.cu).
 int launch_plain_refined(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
                          unsigned long long* d_per_state, const nqb_opts& o, unsigned stack_depth, int device,
                          cudaStream_t s, unsigned* launches, SchedInfo* info,
-                         unsigned long long* d_lane_stats = nullptr);
+                         unsigned long long* d_lane_stats = nullptr, Refined* keep = nullptr);
 
 // A stream of the current device for one call (devmem.cu): an idle one kept from an earlier
 // call, or a new one.  stream_give waits for it and keeps it for later calls; the device it was

@@ -39,18 +39,25 @@ constexpr unsigned kErrBound = 2u;  // checked builds: a push would have passed 
 // nodes: the candidate of a row entered with exactly one candidate, other than the start
 // row).  lane_stats (optional, LANES builds): {lane-steps that placed a queen, lane-step
 // slots issued (32 per warp step)}: their ratio is the search loop's warp execution
-// efficiency in active lanes.
-template <int BLOCK, bool UNIT, bool LANES>
-__global__ void __launch_bounds__(BLOCK) plain_search_kernel(const uint4* __restrict__ states, uint32_t count,
+// efficiency in active lanes.  LEVEL: states, count and board_of come from `level`, for
+// launches whose host has not waited to learn them (N=14 counts 141 -> 128 us); an instance of
+// its own, since the same branch in the others cost the N=19 counts 3%.
+template <int BLOCK, bool UNIT, bool LANES, bool LEVEL>
+__global__ void __launch_bounds__(BLOCK) plain_search_kernel(const uint4* states, uint32_t count,
                                                              unsigned long long* __restrict__ out,
                                                              unsigned long long* __restrict__ per_state,
-                                                             const uint32_t* __restrict__ board_of,
+                                                             const uint32_t* board_of, const ItemLevel* level,
                                                              unsigned long long* __restrict__ lane_stats,
                                                              uint32_t stack_depth) {
     extern __shared__ uint4 stack[];  // [stack_depth + 1][BLOCK]; row 0 holds the sentinels
     constexpr int kStride = BLOCK * 16;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
-    const uint32_t gi = blockIdx.x * BLOCK + tid;
+    if (LEVEL) {
+        states = level->items;
+        count = level->n;
+        board_of = level->board;
+        if (blockIdx.x * BLOCK >= count) return;
+    }
     const uint32_t base0 = (uint32_t)__cvta_generic_to_shared(stack) + tid * 16;
     const uint32_t top = base0 + stack_depth * kStride;  // the lane's last slot
     uint32_t base = base0;
@@ -64,18 +71,25 @@ __global__ void __launch_bounds__(BLOCK) plain_search_kernel(const uint4* __rest
     s.placed = 0;
     uint32_t weight = 0, item = kNoItem;
     bool bad = false;
-    if (gi < count) {
-        const uint4 st = __ldg(states + gi);
+    auto take = [&](uint32_t i) {  // the lane's state: i, if there is one
+        s.sols = 0;
+        s.nodes = 0;
+        if (i >= count) return;
+        base = base0;
+        write_sentinel(base0);
+        const uint4 st = __ldg(states + i);
         if (lane_load(s, st, base) > stack_depth) {
-            bad = true;
+            bad = true;  // skip the state: its search could overrun the stack
             lane_park(s, base);
             s.sols = 0;
             s.nodes = 0;
         } else {
             weight = (st.w >> 16) & 0xFFu;
-            item = gi;
+            item = i;
         }
-    }
+    };
+    uint32_t gi = blockIdx.x * BLOCK + tid;
+    take(gi);
     unsigned long long piece = 0, c = 0, nodes = 0, unit64 = 0, placed64 = 0, rounds = 0;
     uint32_t unit = 0;
     uint32_t epoch = kEpoch;
@@ -91,7 +105,14 @@ __global__ void __launch_bounds__(BLOCK) plain_search_kernel(const uint4* __rest
                 s.sols = 0;
                 item = kNoItem;
             }
-            if (idle == kFull) break;
+            if (idle == kFull) {
+                if (!LEVEL) break;
+                // a level may hold more states than the grid was sized for
+                gi += gridDim.x * BLOCK;
+                if (gi - lane >= count) break;
+                nodes += s.nodes;
+                take(gi);
+            }
             const uint32_t donors = __ballot_sync(kFull, s.sp != base);
             if (donors) share_rows<kStride>(s, base, base0, weight, item, idle, donors, lane);
         }
@@ -157,11 +178,12 @@ __global__ void __launch_bounds__(BLOCK) plain_search_kernel(const uint4* __rest
     }
 }
 
-template <int BLOCK, bool UNIT, bool LANES>
+template <int BLOCK, bool UNIT, bool LANES, bool LEVEL>
 int launch_t(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
-             unsigned long long* d_per_state, const uint32_t* d_board_of, unsigned long long* d_lanes,
+             unsigned long long* d_per_state, const uint32_t* d_board_of, const ItemLevel* d_level,
+             unsigned long long* d_lanes,
              unsigned stack_depth, cudaStream_t stream, unsigned* launches) {
-    auto kern = plain_search_kernel<BLOCK, UNIT, LANES>;
+    auto kern = plain_search_kernel<BLOCK, UNIT, LANES, LEVEL>;
     // Room for the stack (with its sentinel row), and for 4 x (BLOCK/32) reduction words.
     const size_t smem = std::max<size_t>((size_t)(stack_depth + 1) * BLOCK * sizeof(uint4),
                                          4 * (BLOCK / 32) * sizeof(unsigned long long));
@@ -176,7 +198,7 @@ int launch_t(const nqb_state* d_states, uint64_t count, unsigned long long* d_ou
         // without a slot map, a chunk's slots start at its first state
         kern<<<grid, BLOCK, smem, stream>>>(base + off, c, d_out,
                                             d_per_state && !d_board_of ? d_per_state + off : d_per_state,
-                                            d_board_of ? d_board_of + off : nullptr, d_lanes, stack_depth);
+                                            d_board_of ? d_board_of + off : nullptr, d_level, d_lanes, stack_depth);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_status(e);
         if (launches) (*launches)++;
@@ -186,11 +208,17 @@ int launch_t(const nqb_state* d_states, uint64_t count, unsigned long long* d_ou
 
 template <int BLOCK>
 int launch_block(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
-                 unsigned long long* d_per_state, const uint32_t* d_board_of, unsigned long long* d_lanes,
+                 unsigned long long* d_per_state, const uint32_t* d_board_of, const ItemLevel* d_level,
+             unsigned long long* d_lanes,
                  bool count_unit, unsigned stack_depth, cudaStream_t stream, unsigned* launches) {
-    auto launch = d_lanes ? (count_unit ? launch_t<BLOCK, true, true> : launch_t<BLOCK, false, true>)
-                          : (count_unit ? launch_t<BLOCK, true, false> : launch_t<BLOCK, false, false>);
-    return launch(d_states, count, d_out, d_per_state, d_board_of, d_lanes, stack_depth, stream, launches);
+    auto launch = d_level ? (d_lanes ? (count_unit ? launch_t<BLOCK, true, true, true> : launch_t<BLOCK, false, true, true>)
+                                     : (count_unit ? launch_t<BLOCK, true, false, true>
+                                                   : launch_t<BLOCK, false, false, true>))
+                          : (d_lanes ? (count_unit ? launch_t<BLOCK, true, true, false>
+                                                   : launch_t<BLOCK, false, true, false>)
+                                     : (count_unit ? launch_t<BLOCK, true, false, false>
+                                                   : launch_t<BLOCK, false, false, false>));
+    return launch(d_states, count, d_out, d_per_state, d_board_of, d_level, d_lanes, stack_depth, stream, launches);
 }
 
 }  // namespace
@@ -198,21 +226,21 @@ int launch_block(const nqb_state* d_states, uint64_t count, unsigned long long* 
 int launch_plain(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
                  unsigned long long* d_per_state, int block_size, bool count_unit, unsigned stack_depth,
                  cudaStream_t stream, unsigned* launches, unsigned long long* d_lane_stats,
-                 const uint32_t* d_board_of) {
-    if (!d_out || (count && !d_states)) return NQB_E_INVALID;
+                 const uint32_t* d_board_of, const ItemLevel* d_level) {
+    if (!d_out || (count && !d_states && !d_level)) return NQB_E_INVALID;
     if (count == 0) return NQB_OK;
     if (stack_depth == 0) stack_depth = NQB_MAX_N - 1;
     if (stack_depth > NQB_MAX_N) return NQB_E_INVALID;
     if (block_size == 0) block_size = 128;
     switch (block_size) {
         case 64:
-            return launch_block<64>(d_states, count, d_out, d_per_state, d_board_of, d_lane_stats, count_unit, stack_depth,
+            return launch_block<64>(d_states, count, d_out, d_per_state, d_board_of, d_level, d_lane_stats, count_unit, stack_depth,
                                     stream, launches);
         case 128:
-            return launch_block<128>(d_states, count, d_out, d_per_state, d_board_of, d_lane_stats, count_unit, stack_depth,
+            return launch_block<128>(d_states, count, d_out, d_per_state, d_board_of, d_level, d_lane_stats, count_unit, stack_depth,
                                      stream, launches);
         case 256:
-            return launch_block<256>(d_states, count, d_out, d_per_state, d_board_of, d_lane_stats, count_unit, stack_depth,
+            return launch_block<256>(d_states, count, d_out, d_per_state, d_board_of, d_level, d_lane_stats, count_unit, stack_depth,
                                      stream, launches);
         default:
             return NQB_E_INVALID;

@@ -38,16 +38,15 @@ constexpr uint32_t kMinSplitFree = 8;      // items with fewer free columns are 
 constexpr uint32_t kSplitSpread = 3;
 constexpr unsigned kMaxLevels = 4;
 constexpr unsigned kThreads = 256;
-constexpr unsigned kMaxRecords = NQB_MAX_N + kMaxLevels;  // a pool's levels, then the split's
+constexpr unsigned kMaxRecords = kMaxItemLevels;  // a pool's levels, then the split's
+static_assert(kMaxRecords >= NQB_MAX_N + kMaxLevels, "one record a level");
+// With fewer free columns at most, the host does not wait to learn how many items the split made:
+// the search takes the number from the device.  Larger items are worth the wait (12 us), which also
+// tells how deep a stack they need.
+constexpr uint32_t kDeferFree = 12;
 constexpr size_t kHeadBytes = 2048;
 
-struct Level {
-    const uint4* items;
-    const uint32_t* board;      // item -> output slot (nullptr: identity)
-    unsigned long long next;    // items the next level would make of these
-    uint32_t n;
-    uint32_t done;              // levels that split something
-};
+using Level = ItemLevel;
 
 __device__ __forceinline__ uint32_t free_columns(const uint4 s) {
     const uint32_t n = (s.w >> 8) & 0xFFu;
@@ -225,7 +224,7 @@ void Refined::release() {
 
 int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, bool boards, bool unit,
                  unsigned stack_depth, int device, cudaStream_t s, unsigned long long* d_totals,
-                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out) {
+                 unsigned long long* d_board_nodes, unsigned* launches, Refined* out, bool may_defer) {
     out->items = d_items;
     out->board = d_board;
     out->n = n;
@@ -250,6 +249,11 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
     }
     NQB_TRY(cuda_status(cudaGetLastError()));
     if (launches) *launches += 1 + levels;
+    if (may_defer && max_free < kDeferFree) {
+        out->level = lv + levels;
+        out->n = (uint32_t)std::min<uint64_t>((uint64_t)n << (2 * levels), kCapItems);  // about 4 children a level
+        return NQB_OK;
+    }
     Level last;
     NQB_TRY(cuda_status(cudaMemcpyAsync(&last, lv + levels, sizeof(last), cudaMemcpyDeviceToHost, s)));
     NQB_TRY(cuda_status(cudaStreamSynchronize(s)));
@@ -276,8 +280,7 @@ bool small_pool(unsigned n, unsigned depth) {
 }
 
 int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
-                     unsigned* launches, Refined* out, uint64_t* states) {
-    *states = 0;
+                     unsigned* launches, Refined* out, const ItemLevel** all_levels, unsigned* n_levels) {
     int sms = 0;
     NQB_TRY(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)));
     const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;
@@ -299,16 +302,21 @@ int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStre
     }
     NQB_TRY(cuda_status(cudaGetLastError()));
     if (launches) *launches += 1 + all;
+    *all_levels = lv;
+    *n_levels = all + 1;
+    out->stack_depth = max_free > 1 ? max_free - 1 : 1;
+    if (max_free < kDeferFree) {
+        out->level = lv + all;
+        out->n = (uint32_t)std::min<double>(size * 1.25 + 1.0, kCapItems);
+        return NQB_OK;
+    }
     Level rec[kMaxRecords];
     NQB_TRY(cuda_status(cudaMemcpyAsync(rec, lv, (all + 1) * sizeof(Level), cudaMemcpyDeviceToHost, s)));
     NQB_TRY(cuda_status(cudaStreamSynchronize(s)));
     if (rec[depth - 1].done != depth - 1) return NQB_E_RANGE;  // a level of the pool did not fit
-    const Level& last = rec[all];
-    const unsigned split = last.done - (depth - 1);
-    *states = rec[depth - 1].n;
-    out->items = reinterpret_cast<const nqb_state*>(last.items);
-    out->board = nullptr;
-    out->n = last.n;
+    const unsigned split = rec[all].done - (depth - 1);
+    out->items = reinterpret_cast<const nqb_state*>(rec[all].items);
+    out->n = rec[all].n;
     out->stack_depth = max_free > split + 1 ? max_free - split - 1 : 1;
     return NQB_OK;
 }

@@ -261,17 +261,18 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
                              size_t scratch_bytes, unsigned long long* d_out, unsigned long long* d_per_board,
                              unsigned long long* d_per_board_nodes, const nqb_opts& o, unsigned stack_depth,
                              int device, cudaStream_t s, unsigned* launches, SchedInfo* info,
-                             unsigned long long* d_lane_stats) {
+                             unsigned long long* d_lane_stats, Refined* keep) {
     if (!o.model && o.sched_cost == 0) {
         Refined r;
         int st = refine_items(d_items, n, d_board, d_per_board || d_per_board_nodes, false, stack_depth, device, s,
-                              d_out, d_per_board_nodes, launches, &r);
+                              d_out, d_per_board_nodes, launches, &r, keep != nullptr);
         if (!st)
             st = launch_batched(r.items, r.n, nullptr, r.board, d_scratch, scratch_bytes, d_out, d_per_board,
                                 d_per_board_nodes, o.block_size, r.stack_depth, device, s, launches, d_lane_stats, 0,
-                                true);
-        r.release();  // stream-ordered after the kernel that reads the arrays
+                                true, r.level);
         if (info) info->items = r.n;
+        if (keep) *keep = r;
+        else r.release();  // stream-ordered after the kernel that reads the arrays
         return st;
     }
     Schedule sch;
@@ -290,19 +291,21 @@ int launch_batched_scheduled(const nqb_state* d_items, uint32_t n, const uint32_
 
 int launch_plain_refined(const nqb_state* d_states, uint64_t count, unsigned long long* d_out,
                          unsigned long long* d_per_state, const nqb_opts& o, unsigned stack_depth, int device,
-                         cudaStream_t s, unsigned* launches, SchedInfo* info, unsigned long long* d_lane_stats) {
+                         cudaStream_t s, unsigned* launches, SchedInfo* info, unsigned long long* d_lane_stats,
+                         Refined* keep) {
     const bool unit = o.count_unit_nodes != 0;
     if (count > 0xFFFFFFFFull)  // far more than the split is for
         return launch_plain(d_states, count, d_out, d_per_state, o.block_size, unit, stack_depth, s, launches,
                             d_lane_stats);
     Refined r;
     int st = refine_items(d_states, (uint32_t)count, nullptr, d_per_state != nullptr, unit, stack_depth, device, s,
-                          d_out, nullptr, launches, &r);
+                          d_out, nullptr, launches, &r, keep != nullptr);
     if (!st)
         st = launch_plain(r.items, r.n, d_out, d_per_state, o.block_size, unit, r.stack_depth, s, launches,
-                          d_lane_stats, r.board);
-    r.release();
+                          d_lane_stats, r.board, r.level);
     if (info) info->items = r.n;
+    if (keep) *keep = r;
+    else r.release();
     return st;
 }
 
