@@ -51,7 +51,7 @@
 // of that pipe.  The step before it, with a filter for one-column G only, a compare that
 // guarded the stack's bottom, and shifts where this one has multiply-adds, issued 32.2
 // instructions and made 3.6% more steps: 1/16 of the N=20 depth-7 pool (1.18e11 nodes)
-// took 80.2 ms against 72.0 ms.
+// took 80.2 ms against 71.7 ms.
 //
 // Stack bound: a row is pushed only while another candidate remains, and pushed rows are
 // strictly deeper towards the top, so a search from a state with f free columns holds at
@@ -87,17 +87,19 @@ struct StepInfo {
     uint32_t cand0, cand1;
 };
 
+// A stack entry's words lie in the order nc, avail, r, l (here and in the step): with
+// avail, nc, l, r the step runs 1% slower, by the compiler's choice of registers alone.
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "=r"(v.y), "=r"(v.x), "=r"(v.w), "=r"(v.z)
                  : "r"(addr)
                  : "memory");
     return v;
 }
 
 __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
-    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.y), "r"(v.x), "r"(v.w), "r"(v.z)
                  : "memory");
 }
 
@@ -108,7 +110,7 @@ __device__ __forceinline__ void write_sentinel(uint32_t addr) {
 // Gives the sentinel all its bits back.  Every lane may do so at any time: the slot at `base`
 // never holds anything else.
 __device__ __forceinline__ void refresh_sentinel(uint32_t base) {
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(base), "r"(kSentinelAvail) : "memory");
+    asm volatile("st.shared.u32 [%0+4], %1;" ::"r"(base), "r"(kSentinelAvail) : "memory");
 }
 
 // Candidates `a` of a row minus those whose placement leaves the next row empty (see the
@@ -124,7 +126,7 @@ __device__ __forceinline__ uint32_t drop_leaves(uint32_t a, uint32_t nc, uint32_
 #define NQB_STEP(a, n, l, r, A, N, L, R, c, push, count)                                                 \
     "setp.eq.u32 p, " a ", 0;\n\t" /* no candidate left: pop */                                          \
     count                                                                                                \
-    "@p ld.shared.v4.u32 {" a ", " n ", " l ", " r "}, [%4];\n\t"                                        \
+    "@p ld.shared.v4.u32 {" n ", " a ", " r ", " l "}, [%4];\n\t"                                        \
     "@p sub.u32 %4, %4, %10;\n\t"                                                                        \
     "sub.u32 x, " a ", 1;\n\t"                                                                           \
     "not.b32 w, x;\n\t"                                                                                  \
@@ -161,14 +163,14 @@ __device__ __forceinline__ uint32_t drop_leaves(uint32_t a, uint32_t nc, uint32_
 #ifndef NQB_CHECKS
 #define NQB_PUSH(a, n, l, r)       \
     "@t add.u32 %4, %4, %10;\n\t" \
-    "@t st.shared.v4.u32 [%4], {" a ", " n ", " l ", " r "};\n\t"
+    "@t st.shared.v4.u32 [%4], {" n ", " a ", " r ", " l "};\n\t"
 #else
 #define NQB_PUSH(a, n, l, r)                                          \
     "add.u32 x, %4, %10;\n\t" /* the push's slot must not pass top */ \
     "setp.gt.u32 ov, x, %12;\n\t"                                     \
     "and.pred ok, t, !ov;\n\t"                                        \
     "@ok mov.u32 %4, x;\n\t"                                          \
-    "@ok st.shared.v4.u32 [%4], {" a ", " n ", " l ", " r "};\n\t"    \
+    "@ok st.shared.v4.u32 [%4], {" n ", " a ", " r ", " l "};\n\t"    \
     "and.pred ov, t, ov;\n\t"                                         \
     "@ov or.b32 %8, %8, 1;\n\t"
 #endif
