@@ -20,6 +20,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "epoch_order.h"
 #include "mlp.cuh"
 #include "nqb_internal.h"
 
@@ -909,6 +910,7 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
     o.seed = 1;
     if (opts) o = *opts;
     if (o.epochs <= 0 || o.batch <= 0 || o.batch > (1 << 20) || !(o.lr > 0.0f)) return NQB_E_INVALID;
+    EpochOrder order;  // before the scope, which waits for the stream on every way out
     CallScope cs(m->device);
     if (cs.status) return cs.status;
     const uint32_t B = (uint32_t)std::min<uint64_t>(o.batch, count);
@@ -926,22 +928,10 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
     if (!st) st = cuda_status(cudaMemcpyAsync(d_t.p, targets, count * sizeof(float), cudaMemcpyHostToDevice, cs.s));
     if (st) return st;
     features_kernel<<<blocks_for(count * kIn), 256, 0, cs.s>>>(reinterpret_cast<const uint4*>(d_st.p), count, d_X.p);
-    std::vector<uint32_t> perm(count);
-    for (uint64_t i = 0; i < count; ++i) perm[i] = (uint32_t)i;
-    uint64_t rng = o.seed * 0x9E3779B97F4A7C15ull + 1;
-    auto next = [&]() {
-        uint64_t z = (rng += 0x9E3779B97F4A7C15ull);
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        return z ^ (z >> 31);
-    };
+    order.start(count, o.seed);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    auto shuffle = [&] {
-        for (uint64_t i = count - 1; i > 0; --i) std::swap(perm[i], perm[next() % (i + 1)]);  // Fisher-Yates
-    };
-    shuffle();
     for (int ep = 0; ep < o.epochs; ++ep) {
-        st = cuda_status(cudaMemcpyAsync(d_perm.p, perm.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, cs.s));
+        st = cuda_status(cudaMemcpyAsync(d_perm.p, order.current(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, cs.s));
         if (st) return st;
         cudaMemsetAsync(w.loss, 0, sizeof(float), cs.s);
         for (uint64_t off = 0; off < count; off += B) {
@@ -953,12 +943,13 @@ int nqb_model_train(nqb_model* m, const nqb_state* states, const float* targets,
             adam_kernel<<<blocks_for(kParams), 256, 0, cs.s>>>(m->params, w.parts, slots, m->m, m->v, o.lr, b1, b2, eps,
                                                                 c1, c2, m->w1h, m->w2h, w.loss, w.err);
         }
-        if (ep + 1 < o.epochs) shuffle();  // the next epoch's order, while the device works on this one
+        if (ep + 1 < o.epochs) order.prepare();  // while the device works on this epoch
         float l = 0;
         st = cuda_status(cudaMemcpyAsync(&l, w.loss, sizeof(float), cudaMemcpyDeviceToHost, cs.s));
         if (!st) st = w.check(cs.s);
         if (st) return st;
         if (epoch_loss) epoch_loss[ep] = l / (float)count;
+        if (ep + 1 < o.epochs) order.advance();  // check() has waited for the stream
     }
     return cuda_status(cudaStreamSynchronize(cs.s));
 } NQB_ABI_CATCH
