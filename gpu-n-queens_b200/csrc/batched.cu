@@ -379,13 +379,12 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
 template <int BLOCK, bool LANES>
 int launch_batched_t(BatchArgs a, bool refined, int device, cudaStream_t stream, unsigned* launches) {
     const size_t smem = (size_t)(a.stack_depth + 1) * BLOCK * sizeof(uint4);
-    if (smem > 227 * 1024) return NQB_E_RANGE;
+    if (smem > kMaxDynamicSmem) return NQB_E_RANGE;
     auto kern = batched_search_kernel<BLOCK, LANES, false>;
     auto spread = batched_search_kernel<BLOCK, LANES, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(spread, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e);
+    NQB_TRY(allow_dynamic_smem(kern));
+    NQB_TRY(allow_dynamic_smem(spread));
+    cudaError_t e;
     int sms = 0, per_sm = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
         return cuda_status(e);

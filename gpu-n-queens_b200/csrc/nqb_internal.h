@@ -187,6 +187,18 @@ void dev_free(void* p, cudaStream_t s);
 
 int cuda_status(cudaError_t e);
 
+// The most dynamic shared memory a block may have on sm_100.
+constexpr size_t kMaxDynamicSmem = 227 * 1024;
+
+// Lets launches of `kernel` (which has no static shared memory) take up to that much.  The
+// attribute belongs to the function, not to a launch, so every call sets the same value: a
+// launch's own size, set here, would be what another thread's deeper launch then fails on.
+template <class K>
+int allow_dynamic_smem(K* kernel) {
+    return cuda_status(
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem));
+}
+
 // The allocation-failure test hook (nqb_debug_fail_allocation, devmem.cu): true when the
 // allocation being made now is the one chosen to fail.  Every allocation of the library's own
 // code asks it first: device buffers (dev_alloc_bytes, cuda_malloc), pinned host buffers

@@ -187,9 +187,8 @@ int launch_t(const nqb_state* d_states, uint64_t count, unsigned long long* d_ou
     // Room for the stack (with its sentinel row), and for 4 x (BLOCK/32) reduction words.
     const size_t smem = std::max<size_t>((size_t)(stack_depth + 1) * BLOCK * sizeof(uint4),
                                          4 * (BLOCK / 32) * sizeof(unsigned long long));
-    if (smem > 227 * 1024) return NQB_E_RANGE;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e);
+    if (smem > kMaxDynamicSmem) return NQB_E_RANGE;
+    NQB_TRY(allow_dynamic_smem(kern));
     const uint64_t kChunk = 1ull << 30;  // states per launch (grid.x stays < 2^31)
     const uint4* base = reinterpret_cast<const uint4*>(d_states);
     for (uint64_t off = 0; off < count; off += kChunk) {
@@ -199,8 +198,7 @@ int launch_t(const nqb_state* d_states, uint64_t count, unsigned long long* d_ou
         kern<<<grid, BLOCK, smem, stream>>>(base + off, c, d_out,
                                             d_per_state && !d_board_of ? d_per_state + off : d_per_state,
                                             d_board_of ? d_board_of + off : nullptr, d_level, d_lanes, stack_depth);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_status(e);
+        NQB_TRY(cuda_status(cudaGetLastError()));
         if (launches) (*launches)++;
     }
     return NQB_OK;
