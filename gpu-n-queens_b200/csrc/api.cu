@@ -21,6 +21,7 @@ bool state_valid(const nqb_state& s) {
 
 int cuda_status(cudaError_t e) {
     if (e == cudaSuccess) return NQB_OK;
+    cudaGetLastError();  // reported here: the next launch's check must not find it again
     if (e == cudaErrorMemoryAllocation) return NQB_E_NOMEM;
     if (e == cudaErrorNoDevice || e == cudaErrorInvalidDevice || e == cudaErrorInsufficientDriver)
         return NQB_E_NODEVICE;
