@@ -149,6 +149,17 @@ int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s) {
     return cuda_status(cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, s));
 }
 
+int dev_alloc_optional(void** p, size_t bytes, cudaStream_t s) {
+    *p = nullptr;
+    int dev = 0;
+    NQB_TRY(cuda_status(cudaGetDevice(&dev)));
+    cudaMemPool_t pool = nullptr;
+    NQB_TRY(device_pool(dev, &pool));
+    const int st = cuda_status(cudaMallocFromPoolAsync(p, bytes, pool, s));
+    if (st != NQB_OK) *p = nullptr;
+    return st == NQB_E_NOMEM ? NQB_OK : st;
+}
+
 void dev_free(void* p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }

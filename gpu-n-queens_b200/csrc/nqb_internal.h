@@ -101,6 +101,7 @@ int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d
 // into d_totals[1] (unit: the unit ones also into d_totals[2]) and d_board_nodes[board].
 // boards: the items' output slots are needed.  Waits for the stream when it splits, unless
 // may_defer and the items are small: `level` then holds the items and n the number expected.
+// Without device memory to spare for the split, the items stay as they are.
 struct Refined {
     const nqb_state* items = nullptr;
     const uint32_t* board = nullptr;  // item -> output slot (nullptr: identity)
@@ -119,7 +120,8 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
 // size back: for pools of which small_pool(n, depth) says that they fit refine_items' buffers.
 // `out` holds the items to search, in no particular order; counts like refine_items, and defers
 // like it.  *levels (device memory, *n_levels of them): every level from the seeds on; the pool is
-// levels[depth - 1], and did not fit after all unless its `done` is depth - 1.
+// levels[depth - 1], and did not fit after all unless its `done` is depth - 1.  NQB_E_RANGE when
+// that is known before the search, or when the device has no memory to spare for the levels.
 bool small_pool(unsigned n, unsigned depth);
 constexpr unsigned kMaxItemLevels = NQB_MAX_N + 4;
 int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
@@ -184,6 +186,9 @@ int dev_alloc(T** p, size_t bytes, cudaStream_t s) {
     return st;
 }
 void dev_free(void* p, cudaStream_t s);
+// A buffer that the call can do without: *p = nullptr and NQB_OK when the device has no memory for
+// it.  The allocation-failure hook does not count it, since the call it failed would go on.
+int dev_alloc_optional(void** p, size_t bytes, cudaStream_t s);
 
 int cuda_status(cudaError_t e);
 
@@ -200,8 +205,8 @@ int allow_dynamic_smem(K* kernel) {
 }
 
 // The allocation-failure test hook (nqb_debug_fail_allocation, devmem.cu): true when the
-// allocation being made now is the one chosen to fail.  Every allocation of the library's own
-// code asks it first: device buffers (dev_alloc_bytes, cuda_malloc), pinned host buffers
+// allocation being made now is the one chosen to fail.  Every allocation that a call cannot do
+// without asks it first: device buffers (dev_alloc_bytes, cuda_malloc), pinned host buffers
 // (cuda_malloc_host) and host buffers (the pool and state-file arrays).
 bool alloc_fault();
 

@@ -24,6 +24,7 @@
 // 147.5 and 209 ms (same box) at two; at four, calls move within 4% either way.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 #include "nqb_internal.h"
 #include "search_step.cuh"
@@ -33,7 +34,7 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr uint32_t kItemsPerLane = 2;      // levels stop at this many items a resident lane
-constexpr uint32_t kCapItems = 3200000;    // room of each of the two buffers (51 MB)
+constexpr uint32_t kCapItems = 3200000;    // most room of each of the two buffers (51 MB)
 constexpr uint32_t kMinSplitFree = 8;      // items with fewer free columns are a few hundred nodes
 constexpr uint32_t kSplitSpread = 3;
 constexpr unsigned kMaxLevels = 4;
@@ -45,6 +46,8 @@ static_assert(kMaxRecords >= NQB_MAX_N + kMaxLevels, "one record a level");
 // tells how deep a stack they need.
 constexpr uint32_t kDeferFree = 12;
 constexpr size_t kHeadBytes = 2048;
+constexpr uint32_t kSeeds = 16;  // row-0 columns of the left half, at most
+static_assert((NQB_MAX_N + 1) / 2 <= kSeeds, "seed_kernel writes them unasked");
 
 using Level = ItemLevel;
 
@@ -85,12 +88,12 @@ __global__ void first_kernel(const uint4* __restrict__ items, const uint32_t* __
 template <bool COUNT, bool UNIT>
 __global__ void __launch_bounds__(kThreads) level_kernel(const Level* __restrict__ in, Level* __restrict__ out,
                                                          uint4* __restrict__ to, uint32_t* __restrict__ to_board,
-                                                         uint32_t cut, uint32_t next_cut, uint32_t enough,
-                                                         unsigned long long* __restrict__ totals,
+                                                         uint32_t cut, uint32_t next_cut, uint32_t room,
+                                                         uint32_t enough, unsigned long long* __restrict__ totals,
                                                          unsigned long long* __restrict__ board_nodes) {
     const uint32_t n = in->n;
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
-    if (in->next > kCapItems || (COUNT && (n >= enough || in->next == n))) {
+    if (in->next > room || (COUNT && (n >= enough || in->next == n))) {
         if (first) {
             out->items = in->items;
             out->board = in->board;
@@ -191,29 +194,50 @@ unsigned split_levels(uint32_t max_free) {
     return max_free <= kMinSplitFree ? 0 : std::min(kMaxLevels, max_free - kMinSplitFree);
 }
 
-// The buffers of a call's levels: the records, then two item buffers used in turn.
+// The buffers of a call's levels: the records, then two item buffers of `room` items, used in
+// turn.  Room for no more than the levels can make: an N=8 count takes a few KB, only splits of
+// hundreds of thousands of items take all of 2 x 51 MB (2 x 64 MB with output slots).
 struct Levels {
     Level* records;
     uint4* items[2];
     uint32_t* board[2];
-    int take(bool boards, cudaStream_t s, Refined* out) {
+    uint32_t room;
+    // *had = false (and NQB_OK) when the device has no memory to spare for them.
+    int take(uint64_t want, bool boards, cudaStream_t s, Refined* out, bool* had) {
         static_assert(kMaxRecords * sizeof(Level) <= kHeadBytes, "the level records' room");
-        const size_t item_bytes = (size_t)kCapItems * sizeof(uint4);
-        const size_t board_bytes = boards ? (size_t)kCapItems * sizeof(uint32_t) : 0;
-        NQB_TRY(dev_alloc_bytes(&out->buf, kHeadBytes + 2 * (item_bytes + board_bytes), s));
+        room = (uint32_t)std::min<uint64_t>(want, kCapItems);
+        room = (std::max(room, kSeeds) + 15u) & ~15u;  // keeps the buffers aligned
+        size_t bytes = kHeadBytes + 2 * (size_t)room * (sizeof(uint4) + (boards ? sizeof(uint32_t) : 0));
+#ifdef NQB_CHECKS  // tests: less room than the items need; 0: more memory than any device has
+        if (const char* limit = std::getenv("NQB_SPLIT_ROOM")) {
+            const uint32_t most = (uint32_t)std::strtoul(limit, nullptr, 10);
+            if (most == 0) bytes = (size_t)1 << 50;
+            else room = std::min(room, std::max(most, kSeeds) & ~15u);
+        }
+#endif
+        NQB_TRY(dev_alloc_optional(&out->buf, bytes, s));
+        *had = out->buf != nullptr;
+        if (!*had) return NQB_OK;
         out->stream = s;
         char* at = static_cast<char*>(out->buf);
         records = reinterpret_cast<Level*>(at);
         at += kHeadBytes;
         for (int k = 0; k < 2; ++k) {
             items[k] = reinterpret_cast<uint4*>(at);
-            at += item_bytes;
+            at += (size_t)room * sizeof(uint4);
             board[k] = boards ? reinterpret_cast<uint32_t*>(at) : nullptr;
-            at += board_bytes;
+            if (boards) at += (size_t)room * sizeof(uint32_t);
         }
         return NQB_OK;
     }
 };
+
+// The most items that splitting n items of max_free free columns can make: one child a column.
+uint64_t split_bound(uint32_t n, uint32_t max_free, unsigned levels) {
+    uint64_t most = n;
+    for (unsigned k = 0; k < levels && most < kCapItems; ++k) most *= max_free - k;
+    return most;
+}
 
 }  // namespace
 
@@ -236,7 +260,9 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
     const unsigned levels = split_levels(max_free);
     if (n >= enough || levels == 0) return NQB_OK;
     Levels b;
-    NQB_TRY(b.take(boards || d_board, s, out));
+    bool had = false;
+    NQB_TRY(b.take(split_bound(n, max_free, levels), boards || d_board, s, out, &had));
+    if (!had) return NQB_OK;  // no memory to spare: the items are searched as they are
     Level* const lv = b.records;
     NQB_TRY(cuda_status(cudaMemsetAsync(lv, 0, (levels + 1) * sizeof(Level), s)));
     const unsigned grid0 = std::max(1u, std::min((n + kThreads - 1) / kThreads, 4u * (unsigned)sms));
@@ -245,7 +271,7 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
     for (unsigned k = 0; k < levels; ++k) {
         auto kern = unit ? level_kernel<true, true> : level_kernel<true, false>;
         kern<<<4 * sms, kThreads, 0, s>>>(lv + k, lv + k + 1, b.items[k & 1], b.board[k & 1], cut_of(max_free, k),
-                                          cut_of(max_free, k + 1), enough, d_totals, d_board_nodes);
+                                          cut_of(max_free, k + 1), b.room, enough, d_totals, d_board_nodes);
     }
     NQB_TRY(cuda_status(cudaGetLastError()));
     if (launches) *launches += 1 + levels;
@@ -286,8 +312,18 @@ int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStre
     const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;
     const uint32_t max_free = n - depth;
     const unsigned levels = split_levels(max_free), all = depth - 1 + levels;
+    // Room for the largest level.  Over all (n, depth) that small_pool lets through the estimate is
+    // 1.0 to 8 times what the levels make (replayed on the CPU); a split stops at `enough` items.
+    double most = 0.0, level = (n + 1) / 2;
+    for (unsigned k = 0; k <= all; ++k) {
+        most = std::max(most, level);
+        if (k >= depth - 1 && level >= 2.0 * enough) break;
+        level *= children_estimate(n, k + 1);
+    }
     Levels b;
-    NQB_TRY(b.take(false, s, out));
+    bool had = false;
+    NQB_TRY(b.take((uint64_t)std::min<double>(most, kCapItems) + 64, false, s, out, &had));
+    if (!had) return NQB_E_RANGE;  // no memory to spare: the caller builds the pool level by level
     Level* const lv = b.records;
     auto cut = [&](unsigned k) { return k < depth - 1 ? 0u : cut_of(max_free, k - (depth - 1)); };
     seed_kernel<<<1, 32, 0, s>>>(n, all ? cut(0) : 0u, b.items[1], lv);
@@ -296,8 +332,8 @@ int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStre
         auto kern = k < depth - 1 ? level_kernel<false, false>
                                   : unit ? level_kernel<true, true> : level_kernel<true, false>;
         const unsigned grid = (unsigned)std::min(4.0 * sms, size / kThreads + 1.0);
-        kern<<<grid, kThreads, 0, s>>>(lv + k, lv + k + 1, b.items[k & 1], nullptr, cut(k), cut(k + 1), enough,
-                                       d_totals, nullptr);
+        kern<<<grid, kThreads, 0, s>>>(lv + k, lv + k + 1, b.items[k & 1], nullptr, cut(k), cut(k + 1), b.room,
+                                       enough, d_totals, nullptr);
         size *= children_estimate(n, k + 1);
     }
     NQB_TRY(cuda_status(cudaGetLastError()));

@@ -139,14 +139,17 @@ int nqb_device_check(int device);
 /* Device buffers of a call (the pool, its level buffers, scratch) come from the library's
  * own stream-ordered memory pool on that device and stay cached for the next call instead
  * of being unmapped, and up to 16 idle streams are kept for the next calls; this returns the
- * cached memory of `device` to the driver and destroys its idle streams. */
+ * cached memory of `device` to the driver and destroys its idle streams.  A count or a batch
+ * with few states also splits them in two buffers of that pool: a few KB for the smallest calls,
+ * 128 MB at most; when the device has no room for them, the call goes on without the split. */
 int nqb_trim_device_memory(int device);
 
 /* Test hook for the error paths: makes one allocation of the library fail as if memory had
  * run out.  after >= 0: the library's next `after` allocations succeed and the one after
  * them fails (once; the hook is then off); after < 0 turns the hook off.  Counted are the
  * library's own device buffers, pinned host buffers and host arrays (pools, state-file
- * placements), from every thread; allocations inside the C++ standard library are not.
+ * placements), from every thread; allocations inside the C++ standard library are not, nor the
+ * buffers of the split of small launches, without which a call goes on.
  * Returns the countdown it replaces: -1 when the hook was off or has fired, else the number
  * of allocations that were still to succeed.  A call whose allocation fails returns
  * NQB_E_NOMEM, releases what it had allocated and leaves the library usable; no entry point
