@@ -71,6 +71,12 @@ constexpr uint32_t kEpoch = (1u << 27) / kUnroll;  // rounds between folds: 31 n
 // 18.40 ms).
 constexpr uint32_t kDonateEvery = 128, kDonateEveryPlenty = 512;
 constexpr uint64_t kPlentyItems = 4;
+// Refined items get a grid for their number while they have at most this many free columns, else the
+// wave and a share of the queue each (SPREAD).  Whole calls, small grid against wave: 256 boards of
+// n 8-12 (8 columns after the split) 123 / 149 us; one board with 9 columns left (n=20, 7 queens) 137 /
+// 180 us, 10 left (n=20, 6 queens) 177 / 193 us and 64 such boards 306 / 278 us, 11 left (n=20, 5
+// queens) 334 / 225 us, 13 left (n=20, 3 queens) 5.57 / 2.02 ms and (n=24, 7 queens) 2.12 / 0.53 ms.
+constexpr uint32_t kSmallFree = 10;
 
 // Error flags written to out[3].
 constexpr unsigned long long kErrStack = 1ull;  // an item needed a deeper stack than provided
@@ -394,15 +400,16 @@ int launch_batched_t(BatchArgs a, bool refined, int device, cudaStream_t stream,
     const uint64_t need = ((uint64_t)a.n_items + BLOCK - 1) / BLOCK;
     // One wave of blocks; with stealing, fewer items than lanes still fill the whole GPU.
     const uint64_t wave = (uint64_t)sms * per_sm;
-    // Refined items that are few are small: a block for every 32 of them, as every warp of the
-    // wave costs the launch three atomics on shared words (256 boards of n 8-12, whole call:
-    // 149 -> 123 us).
-    const uint64_t most = refined ? ((uint64_t)a.n_items + 31) / 32 : a.ring_cap ? wave : need;
+    // Few refined items with at most kSmallFree free columns are little work: a block for every 32 of
+    // them, as every warp of the wave costs the launch three atomics on shared words.  A few large
+    // boards leave items of more columns (the split ends after its last level): they get the wave.
+    const bool small = refined && (a.level || a.stack_depth < kSmallFree);
+    const uint64_t most = small ? ((uint64_t)a.n_items + 31) / 32 : a.ring_cap ? wave : need;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(wave, most));
     const uint64_t lanes = (uint64_t)grid * BLOCK;
     a.donate_every = a.n_items >= kPlentyItems * lanes ? kDonateEveryPlenty : kDonateEvery;
     // (the large launches' instance reads no level: the branch in their loop cost 0.4%)
-    if (a.level || (a.ring_cap && !refined && a.n_items < lanes))
+    if (a.level || (a.ring_cap && !small && a.n_items < lanes))
         spread<<<grid, BLOCK, smem, stream>>>(a);
     else
         kern<<<grid, BLOCK, smem, stream>>>(a);

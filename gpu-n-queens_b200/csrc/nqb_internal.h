@@ -87,8 +87,8 @@ uint32_t batched_ring_slots(size_t scratch_bytes);
 // d_order (optional): queue position -> item; d_board_of (optional): item -> output slot.
 // d_out: {weighted count, nodes, 0, error flags}.  d_lane_stats as for launch_plain.
 // wait_limit: polls without progress before a wait of the work stealing gives up (0 =
-// kBatchedWaitLimit).  refined: the items have been through refine_items, so few of them means
-// little work.  d_level as for launch_plain.
+// kBatchedWaitLimit).  refined: the items have been through refine_items, so few of them that are
+// small (by stack_depth) mean little work.  d_level as for launch_plain; its items are small.
 int launch_batched(const nqb_state* d_items, uint32_t n_items, const uint32_t* d_order, const uint32_t* d_board_of,
                    void* d_scratch, size_t scratch_bytes, unsigned long long* d_out,
                    unsigned long long* d_per_board, unsigned long long* d_per_board_nodes, int block_size,
