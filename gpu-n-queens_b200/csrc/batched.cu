@@ -62,14 +62,23 @@ constexpr int kUnroll = NQB_BATCHED_UNROLL;
 constexpr int kRefresh = 24;  // steps between refreshes of the lanes' sentinels
 static_assert(kRefresh <= kMaxParkedSteps, "a parked lane would pop past its sentinel");
 constexpr uint32_t kEpoch = (1u << 27) / kUnroll;  // rounds between folds: 31 nodes x kUnroll x kEpoch < 2^32
-// Rounds between a busy warp's looks at the hungry count.  A look that finds hungry warps gives
-// pieces away that are often small, so looking often costs more than the waits it saves: with
-// few items a lane every 128 rounds is best (1/16 of the N=20 depth-6 pool, one item a lane:
-// 16 / 32 / 64 / 128 / 512 rounds 91.3 / 88.4 / 86.0 / 84.4 / 85.9 ms; the N=18 depth-5 pool
-// 28.2 / 26.7 / 26.3 / 26.4 / 29.0 ms), and from kPlentyItems a lane on the queue itself keeps
-// the warps busy to the end (N=18 at depth 6 16 / 64 / 128 / 512 rounds 18.45 / 18.59 / 18.65 /
-// 18.40 ms).
+// Rounds after which a busy warp gives rows to hungry ones.  Pieces given away are often small, so
+// giving often costs more than the waits it saves: with few items a lane every 128 rounds is best
+// (1/16 of the N=20 depth-6 pool, one item a lane: 16 / 32 / 64 / 128 / 512 rounds 91.3 / 88.4 / 86.0 /
+// 84.4 / 85.9 ms; the N=18 depth-5 pool 28.2 / 26.7 / 26.3 / 26.4 / 29.0 ms), and from kPlentyItems a
+// lane on the queue itself keeps the warps busy to the end (N=18 at depth 6 16 / 64 / 128 / 512 rounds
+// 18.45 / 18.59 / 18.65 / 18.40 ms).
 constexpr uint32_t kDonateEvery = 128, kDonateEveryPlenty = 512;
+// A long subtree at the end of an uneven queue cannot wait for that, since each gift at most doubles
+// the warps that work on it.  Every kLook rounds (a load and a vote, not measurable) a warp looks at
+// the hungry count, and once half of the warps are hungry it gives after kHotRounds x (warps / hungry)
+// rounds.  Against 128 or 512 rounds throughout: 700,000 boards of n 10-12 and one n=20 board with 3
+// queens 40.1 -> 12.8 ms, 400,000 and one with 4 queens 8.5 -> 5.5 ms, 3,000 boards of n 12-17 5.9 ->
+// 5.75 ms.  Even pools: N=14 at depth 4 0.173 -> 0.160 ms, N=16 at depth 5 0.63 ms, N=17 at depth 5
+// 3.05 -> 3.09 ms, N=18 at depth 6 18.4 ms, N=19 at depth 6 146.7 -> 144.3 ms.  After 16 rounds the
+// second takes 4.7 ms, but N=16 at depth 5 0.645 ms.
+constexpr uint32_t kLook = 16, kHotRounds = 32;
+static_assert(kDonateEvery % kLook == 0 && kDonateEveryPlenty % kLook == 0, "rounds are checked every kLook");
 constexpr uint64_t kPlentyItems = 4;
 // Refined items get a grid for their number while they have at most this many free columns, else the
 // wave and a share of the queue each (SPREAD).  Whole calls, small grid against wave: 256 boards of
@@ -95,7 +104,8 @@ struct BatchArgs {
     uint4* ring;                          // steal ring (2 x uint4 per slot), turn words zero at launch
     uint32_t ring_cap;                    // slots, a power of two; 0 = no stealing across warps
     uint32_t ring_shift;                  // log2(ring_cap)
-    uint32_t donate_every;                // rounds between looks at the hungry count
+    uint32_t donate_every;                // rounds after which a busy warp gives to hungry ones
+    uint32_t warps;                       // of the launch
     uint32_t wait_limit;                  // polls without progress before a wait gives up
     unsigned long long* out;              // {weighted count, nodes, 0, error flags}
     unsigned long long* per_board;        // optional: weighted count per board
@@ -303,17 +313,20 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
         // Publish rows for hungry warps: while the ring holds fewer than 32 rows per hungry
         // warp (and at most half its slots), lanes with pending rows give their bottom row.
         // A warp whose lanes are all busy looks at the hungry count too: it need not have
-        // seen the item queue run dry itself (hungry warps exist only once it has).  The tail
+        // seen the item queue run dry itself (hungry warps exist only once it has).  When a warp
+        // gives: kDonateEvery, kLook.  The tail
         // only moves by a compare-and-swap against the snapshot the room was computed from,
         // so the ring never holds more than half its slots and a producer never waits a lap.
-        if (a.ring_cap && ++rounds == a.donate_every) {
-            rounds = 0;
+        if (a.ring_cap && ++rounds % kLook == 0) {
+            const bool due = rounds >= a.donate_every;
             const uint32_t donors = __ballot_sync(kFull, s.sp != base);
             if (donors) {
-                uint32_t k = 0, t0 = 0;
+                uint32_t k = 0, t0 = 0, tried = 0;
                 if (lane == 0) {
                     const uint32_t g = ld_relaxed(hungry_warps);
-                    if (g) {
+                    const bool hot = 2 * g >= a.warps && rounds * g >= kHotRounds * a.warps;
+                    if (g && (due || hot)) {
+                        tried = 0x100u;
                         const unsigned long long ht =
                             ld_relaxed64(reinterpret_cast<const unsigned long long*>(ring_head));
                         const uint32_t h = (uint32_t)ht, t = (uint32_t)(ht >> 32);
@@ -325,8 +338,10 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
                         }
                     }
                 }
-                k = __shfl_sync(kFull, k, 0);
+                k = __shfl_sync(kFull, k | tried, 0);
                 t0 = __shfl_sync(kFull, t0, 0);
+                if (k) rounds = 0;
+                k &= 0xFFu;
                 const uint32_t rd = __popc(donors & lt_mask);
                 if (((donors >> lane) & 1u) && rd < k) {
                     const uint32_t idx = t0 + rd;
@@ -344,6 +359,7 @@ __global__ void __launch_bounds__(BLOCK) batched_search_kernel(const BatchArgs a
                     }
                 }
             }
+            if (due) rounds = 0;
         }
         if (--epoch == 0) {  // fold lane counters before they can wrap
             piece_sols += s.sols;
@@ -407,6 +423,7 @@ int launch_batched_t(BatchArgs a, bool refined, int device, cudaStream_t stream,
     const uint64_t most = small ? ((uint64_t)a.n_items + 31) / 32 : a.ring_cap ? wave : need;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(wave, most));
     const uint64_t lanes = (uint64_t)grid * BLOCK;
+    a.warps = (uint32_t)(lanes / 32);
     a.donate_every = a.n_items >= kPlentyItems * lanes ? kDonateEveryPlenty : kDonateEvery;
     // (the large launches' instance reads no level: the branch in their loop cost 0.4%)
     if (a.level || (a.ring_cap && !small && a.n_items < lanes))
