@@ -113,11 +113,11 @@ struct OwnPool {
 
 // Solves `count` states already on the device (d_states, stack bound `depth`), or those of
 // `pool`, with the form o.form; fills totals {count, nodes, unit, err} and optional per-state
-// results.  e_start is recorded before any H2D copy so that h2d_ms covers it.  NQB_E_RANGE
-// with a pool: it is larger than small_pool took it for.
+// results.  e_start and e_copied (or neither) stand around the copy of the states, for h2d_ms.
+// NQB_E_RANGE with a pool: it is larger than small_pool took it for.
 int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, unsigned depth, const nqb_opts& o,
                         unsigned long long totals[4], uint64_t* per_state, nqb_stats* st,
-                        uint64_t* per_state_nodes, cudaEvent_t e_start, OwnPool* pool = nullptr) {
+                        uint64_t* per_state_nodes, cudaEvent_t e_start, cudaEvent_t e_copied, OwnPool* pool = nullptr) {
     const bool batched = o.form == NQB_FORM_BATCHED;
     if (o.form != NQB_FORM_PLAIN && !batched) return NQB_E_INVALID;
     if (batched && count > (1ull << 31)) return NQB_E_RANGE;
@@ -149,10 +149,9 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
         NQB_TRY(sc.event(&e0));
         NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
         const int s = small_pool_items(pool->n, pool->depth, o.count_unit_nodes && !batched, sc.device, sc.stream,
-                                       d_out, &launches, &own, &d_levels, &n_levels);
+                                       d_out, &launches, &own, &d_levels, &n_levels, e1);
         sc.hold(own.buf);
         NQB_TRY(s);
-        NQB_TRY(cuda_status(cudaEventRecord(e1, sc.stream)));
         sched.items = own.n;
         if (batched)
             NQB_TRY(launch_batched(own.items, own.n, nullptr, nullptr, d_out + 8, kBatchedScratchBytes, d_out, nullptr,
@@ -206,7 +205,7 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     if (totals[3]) return NQB_E_DEVICE;
     if (st) {
         float h2d = 0, ker = 0;
-        if (e_start) cudaEventElapsedTime(&h2d, e_start, e1);
+        if (e_start) cudaEventElapsedTime(&h2d, e_start, e_copied);
         cudaEventElapsedTime(&ker, e1, e2);
         st->states = count;
         st->nodes = totals[1];
@@ -266,11 +265,13 @@ int solve_host_states(Scope& sc, const nqb_state* states, uint64_t count, const 
     }
     nqb_state* d_states = nullptr;
     NQB_TRY(sc.alloc(&d_states, count * sizeof(nqb_state)));
-    cudaEvent_t e0;
+    cudaEvent_t e0, e_copied;
     NQB_TRY(sc.event(&e0));
+    NQB_TRY(sc.event(&e_copied));
     NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
     NQB_TRY(cuda_status(
         cudaMemcpyAsync(d_states, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, sc.stream)));
+    NQB_TRY(cuda_status(cudaEventRecord(e_copied, sc.stream)));
     if (on_device) {
         unsigned *d_seen = nullptr, seen[2] = {0, 0};
         NQB_TRY(sc.alloc(&d_seen, sizeof(seen)));
@@ -283,7 +284,7 @@ int solve_host_states(Scope& sc, const nqb_state* states, uint64_t count, const 
         if (seen[0]) return NQB_E_INVALID;
         depth = seen[1] > 1 ? seen[1] - 1 : 1;
     }
-    return solve_device_states(sc, d_states, count, depth, o, totals, per_state, st, per_state_nodes, e0);
+    return solve_device_states(sc, d_states, count, depth, o, totals, per_state, st, per_state_nodes, e0, e_copied);
 }
 
 void* aligned_host_alloc(size_t bytes) {
@@ -409,7 +410,7 @@ int nqb_count_ex(unsigned n, unsigned depth, const nqb_opts* opts, uint64_t* cou
         OwnPool own{n, depth, 0.0};
         int s = NQB_E_RANGE;
         if (small_pool(n, depth) && (o.form == NQB_FORM_PLAIN || (!o.model && o.sched_cost == 0))) {
-            s = solve_device_states(sc, nullptr, 0, 0, o, totals, nullptr, stats, nullptr, nullptr, &own);
+            s = solve_device_states(sc, nullptr, 0, 0, o, totals, nullptr, stats, nullptr, nullptr, nullptr, &own);
             gen_ms = own.gen_ms;
         }
         if (s == NQB_E_RANGE) {
@@ -422,7 +423,7 @@ int nqb_count_ex(unsigned n, unsigned depth, const nqb_opts* opts, uint64_t* cou
             NQB_TRY(generate_pool_device(n, depth, sc.stream, &d_pool, &cnt));
             cudaEventRecord(g1, sc.stream);
             s = solve_device_states(sc, d_pool, cnt, n - depth - 1 > 0 ? n - depth - 1 : 1, o, totals, nullptr, stats,
-                                    nullptr, nullptr);
+                                    nullptr, nullptr, nullptr);
             dev_free(d_pool, sc.stream);
             float g = 0.0f;
             if (s == NQB_OK) cudaEventElapsedTime(&g, g0, g1);

@@ -122,10 +122,12 @@ int refine_items(const nqb_state* d_items, uint32_t n, const uint32_t* d_board, 
 // like it.  *levels (device memory, *n_levels of them): every level from the seeds on; the pool is
 // levels[depth - 1], and did not fit after all unless its `done` is depth - 1.  NQB_E_RANGE when
 // that is known before the search, or when the device has no memory to spare for the levels.
+// pool_built is recorded between the pool's levels and the split's.
 bool small_pool(unsigned n, unsigned depth);
 constexpr unsigned kMaxItemLevels = NQB_MAX_N + 4;
 int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
-                     unsigned* launches, Refined* out, const ItemLevel** levels, unsigned* n_levels);
+                     unsigned* launches, Refined* out, const ItemLevel** levels, unsigned* n_levels,
+                     cudaEvent_t pool_built);
 
 // Items after learned scheduling: the caller's arrays, or split / ordered device copies
 // owned by the schedule until release() (stream-ordered frees).

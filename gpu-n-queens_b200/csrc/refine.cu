@@ -306,7 +306,8 @@ bool small_pool(unsigned n, unsigned depth) {
 }
 
 int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStream_t s, unsigned long long* d_totals,
-                     unsigned* launches, Refined* out, const ItemLevel** all_levels, unsigned* n_levels) {
+                     unsigned* launches, Refined* out, const ItemLevel** all_levels, unsigned* n_levels,
+                     cudaEvent_t pool_built) {
     int sms = 0;
     NQB_TRY(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)));
     const uint32_t enough = kItemsPerLane * (uint32_t)sms * 1152;
@@ -329,6 +330,7 @@ int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStre
     seed_kernel<<<1, 32, 0, s>>>(n, all ? cut(0) : 0u, b.items[1], lv);
     double size = (n + 1) / 2;  // of the level's input, for the grid
     for (unsigned k = 0; k < all; ++k) {
+        if (k == depth - 1) NQB_TRY(cuda_status(cudaEventRecord(pool_built, s)));
         auto kern = k < depth - 1 ? level_kernel<false, false>
                                   : unit ? level_kernel<true, true> : level_kernel<true, false>;
         const unsigned grid = (unsigned)std::min(4.0 * sms, size / kThreads + 1.0);
@@ -336,6 +338,7 @@ int small_pool_items(unsigned n, unsigned depth, bool unit, int device, cudaStre
                                        enough, d_totals, nullptr);
         size *= children_estimate(n, k + 1);
     }
+    if (all == depth - 1) NQB_TRY(cuda_status(cudaEventRecord(pool_built, s)));
     NQB_TRY(cuda_status(cudaGetLastError()));
     if (launches) *launches += 1 + all;
     *all_levels = lv;

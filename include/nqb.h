@@ -107,9 +107,10 @@ typedef struct nqb_stats {
     uint64_t states;     /* pool states (or boards) solved                         */
     uint64_t nodes;      /* queen placements at rows >= each state's start row     */
     uint64_t unit_nodes; /* of which unit-row propagations; UINT64_MAX if not counted */
-    double gen_ms;       /* host pool generation                                   */
-    double h2d_ms;       /* host->device copy of the pool                          */
-    double kernel_ms;    /* device time of the search kernels (CUDA events)        */
+    double gen_ms;       /* pool generation, on the device or (host_pool) the host  */
+    double h2d_ms;       /* host->device copy of the states                        */
+    double kernel_ms;    /* device time of the search (CUDA events), with the splitting and
+                            ordering of its items and any wait for their number     */
     double wall_ms;      /* whole call                                             */
     uint32_t pregen_depth;
     uint32_t kernel_launches;
