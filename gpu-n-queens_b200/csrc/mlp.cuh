@@ -28,10 +28,6 @@ constexpr float kGeluA = 0.044715f;
 __device__ __forceinline__ float gelu(float x) {
     return 0.5f * x * (1.0f + tanhf(kGeluC * (x + kGeluA * x * x * x)));
 }
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float th = tanhf(kGeluC * (x + kGeluA * x * x * x));
-    return 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluA * x * x);
-}
 
 __host__ __device__ __forceinline__ uint32_t popc32(uint32_t v) {
 #ifdef __CUDA_ARCH__
@@ -79,10 +75,6 @@ __host__ __device__ __forceinline__ float feature(const uint4 st, int j) {
         }
         default: return 0.0f;
     }
-}
-
-__device__ __forceinline__ uint32_t pack_half2(__half lo, __half hi) {
-    return (uint32_t)__half_as_ushort(lo) | ((uint32_t)__half_as_ushort(hi) << 16);
 }
 
 }  // namespace mlp
