@@ -113,7 +113,7 @@ struct OwnPool {
 
 // Solves `count` states already on the device (d_states, stack bound `depth`), or those of
 // `pool`, with the form o.form; fills totals {count, nodes, unit, err} and optional per-state
-// results.  e_start and e_copied (or neither) stand around the copy of the states, for h2d_ms.
+// results.  h2d_ms is the time from e_start (if any) to e_copied, or to the search without one.
 // NQB_E_RANGE with a pool: it is larger than small_pool took it for.
 int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, unsigned depth, const nqb_opts& o,
                         unsigned long long totals[4], uint64_t* per_state, nqb_stats* st,
@@ -205,7 +205,7 @@ int solve_device_states(Scope& sc, const nqb_state* d_states, uint64_t count, un
     if (totals[3]) return NQB_E_DEVICE;
     if (st) {
         float h2d = 0, ker = 0;
-        if (e_start) cudaEventElapsedTime(&h2d, e_start, e_copied);
+        if (e_start) cudaEventElapsedTime(&h2d, e_start, e_copied ? e_copied : e1);
         cudaEventElapsedTime(&ker, e1, e2);
         st->states = count;
         st->nodes = totals[1];
@@ -265,14 +265,14 @@ int solve_host_states(Scope& sc, const nqb_state* states, uint64_t count, const 
     }
     nqb_state* d_states = nullptr;
     NQB_TRY(sc.alloc(&d_states, count * sizeof(nqb_state)));
-    cudaEvent_t e0, e_copied;
+    cudaEvent_t e0, e_copied = nullptr;
     NQB_TRY(sc.event(&e0));
-    NQB_TRY(sc.event(&e_copied));
     NQB_TRY(cuda_status(cudaEventRecord(e0, sc.stream)));
     NQB_TRY(cuda_status(
         cudaMemcpyAsync(d_states, states, count * sizeof(nqb_state), cudaMemcpyHostToDevice, sc.stream)));
-    NQB_TRY(cuda_status(cudaEventRecord(e_copied, sc.stream)));
     if (on_device) {
+        NQB_TRY(sc.event(&e_copied));  // in this branch only: an event costs a small call 3 us
+        NQB_TRY(cuda_status(cudaEventRecord(e_copied, sc.stream)));
         unsigned *d_seen = nullptr, seen[2] = {0, 0};
         NQB_TRY(sc.alloc(&d_seen, sizeof(seen)));
         NQB_TRY(cuda_status(cudaMemsetAsync(d_seen, 0, sizeof(seen), sc.stream)));
