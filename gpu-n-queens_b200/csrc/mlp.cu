@@ -165,9 +165,9 @@ __device__ __forceinline__ void feature_chunk(const uint4 s, uint32_t j, uint32_
 // is bounded; on a timeout the block sets the error word and leaves, freeing its tensor memory
 // on the way out.
 //
-// What bounds it: the tanh of 256 activations and the features of each row, and the waits of a
-// tile's chain; two blocks an SM take turns at it.  300,000 rows: 119 us
-// (190 us with 4 warps a block, each thread a whole row).
+// What bounds it: instruction issue (71% of the slots; ALU pipe 43%, FMA 36%, XU 34%) for the
+// features and the tanh of 256 activations of each row; two blocks an SM take turns at the waits of a
+// tile's chain.  300,000 rows: 119 us (190 us with 4 warps a block, each thread a whole row).
 constexpr uint32_t kPredictThreads = 512;
 constexpr uint32_t kPredictFloats = 3 * kH + 4 + 4 * kTileRows;  // b1 b2 w3 b3 | y partials
 constexpr size_t kPredictSmem = 1024 /* alignment slack */ + 3 * kOpBytes + kPredictFloats * sizeof(float) + 16;
@@ -304,11 +304,11 @@ __global__ void __launch_bounds__(kPredictThreads, 2)
 // optimizer kernel adds the slots up in a fixed order: no atomics, and two runs on the same
 // inputs give the same weights.
 //
-// What bounds it: the tanh of 256 activations a row and the waits of one tile's chain of
-// products (32 blocks at the default batch of 4096).  As 5 GEMMs, 10 elementwise or reducing
-// kernels and 2 gathers through global memory the step took 230 us on the device (two thirds of
-// it in the GEMMs, 20-50 us each); two epochs over 65,536 samples, whole call: 6.75 ms before,
-// 1.51 ms now.
+// What bounds it: the latency of one tile's chain of products, loads and barriers, 29 us a step at the
+// default batch of 4096; its 32 blocks leave 116 SMs idle and issue in 28% of their own slots.  As 5
+// GEMMs, 10 elementwise or reducing kernels and 2 gathers through global memory the step took 230 us
+// on the device (two thirds of it in the GEMMs, 20-50 us each); two epochs over 65,536 samples, whole
+// call: 6.75 ms before, 1.51 ms now.
 constexpr uint32_t kTrainThreads = 512;
 constexpr uint32_t kTrainTmem = 512;
 constexpr uint32_t kTrainFloats = 3 * kH + 4 + 4 * kTileRows + kTileRows;  // b1 b2 w3 b3 | y partials | dy

@@ -46,7 +46,7 @@
 //
 // What bounds a step: instruction issue and the shared-memory pipe (an LDS.128 and an
 // STS.128, 4 wavefronts each whenever some lane of each 8 takes part) together.  At N=19,
-// depth 7 a warp step issues 28.5 instructions (84% of the issue slots) and keeps the
+// depth 7 a warp step issues 28.3 instructions (84% of the issue slots) and keeps the
 // shared-memory pipe 93% busy; with five instructions taken out it runs 8% faster, at 98%
 // of that pipe.  The step before it, with a filter for one-column G only, a compare that
 // guarded the stack's bottom, and shifts where this one has multiply-adds, issued 32.2
